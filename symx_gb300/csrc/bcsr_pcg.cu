@@ -145,8 +145,14 @@ BcsrPcgResult run_bcsr_pcg(int n_blocks, const int32_t* row_ptr, const int32_t* 
     }
 
     launch_pcg_init_rhs<T>(B, b, s);
+    ResidentPlan resident;
+    const bool one_launch = plan_pcg_resident<T>(n_blocks, nnzb, resident);
+    if (one_launch) {
+        launch_pcg_resident<T>(B, resident, s);
+        ck(cudaMemcpyAsync(&h, hdr, sizeof(Header), cudaMemcpyDeviceToHost, s), "read state");
+    }
     int launched = 0, chunk = 8;
-    while (true) {
+    while (!one_launch) {
         for (int k = 0; k < chunk; ++k) launch_pcg_iteration<T>(B, launched + k, s);
         launched += chunk;
         ck(cudaMemcpyAsync(&h, hdr, sizeof(Header), cudaMemcpyDeviceToHost, s), "read state");
@@ -156,6 +162,7 @@ BcsrPcgResult run_bcsr_pcg(int n_blocks, const int32_t* row_ptr, const int32_t* 
     }
     launch_rows4_to_vec3<T>(n_blocks, B.x, x, s);
     ck(cudaStreamSynchronize(s), "synchronize");
+    if (h.st.wait_failed) throw std::runtime_error("symx_gb300 bcsr_pcg: a bounded wait in the PCG kernels gave up");
     res.converged = h.st.converged;
     res.iterations = h.st.iteration;
     res.indefinite = h.st.indefinite;

@@ -20,15 +20,17 @@
 //    primary context) looks the address up again, so a cached address never outlives the
 //    context it belongs to.  If that first call is the set-up step of a program that later
 //    captures streams, it must come before any stream capture.
-//  * Device assumption: the reduction partials have room for kNoAllocPartials = 2,048
-//    per-block sums.  The widest PCG launch is one block of 256 threads per resident slot,
-//    i.e. SMs x resident blocks per SM (GB300: 152 x 8 = 1,216).  A device with room for more
-//    resident blocks than 2,048 is refused by run_bcsr_pcg before any launch.
+//  * Device assumption: the reduction partials have room for kNoAllocPartials = 4,096
+//    per-block sums (the resident PCG's exchange words need 62.5 KB of them).  The widest
+//    other PCG launch is one block of 256 threads per resident slot, i.e. SMs x resident
+//    blocks per SM (GB300: 152 x 8 = 1,216).  A device with room for more resident blocks
+//    than 4,096 is refused by run_bcsr_pcg before any launch.
 //  * What must be zero when the kernels start: the eight completion tickets of the
 //    reductions and the missing-diagonal counter.  Every call clears them on its stream
 //    (cudaMemsetAsync / cudaMemcpyAsync into the array) before its first kernel.  Everything
 //    else in the array is written before it is read.
 #include "bcsr_pcg.h"
+#include "kernels.cuh"
 
 #include <cstdint>
 #include <mutex>
@@ -38,9 +40,10 @@
 namespace {
 
 constexpr int kNoAllocMaxBlocks = 65536;
-// Room for the per-block partial sums of the widest PCG launch (152 SMs x 8 blocks of 256
-// threads = 1,216 on GB300); run_bcsr_pcg checks the real grid against it.
-constexpr unsigned kNoAllocPartials = 2048;
+// Room for the resident PCG's exchange words (kResidentPartials) and the per-block partial sums of
+// the widest PCG launch (152 SMs x 8 blocks of 256 threads = 1,216 on GB300); run_bcsr_pcg checks
+// the real grid against it.
+constexpr unsigned kNoAllocPartials = symxg::kResidentPartials;
 constexpr size_t kNoAllocBytes = symxg::bcsr_pcg_workspace_size(kNoAllocMaxBlocks, kNoAllocPartials, sizeof(float));
 
 }  // namespace

@@ -222,6 +222,24 @@ StagedSizes plan_staged_spmv(int n_blocks, const int32_t* row_ptr_host, PcgBuffe
 // chunk counters of its dynamically scheduled product passes.
 void launch_pcg_solve_persistent(const PcgBuffers<float>& B, cudaStream_t s);
 
+// All PCG iterations in one cooperative launch with the matrix rows held in shared memory
+// (k_pcg_resident), float or double, strided values: for systems whose vectors fit in the SMs'
+// shared memory together.  plan_pcg_resident returns false when they do not (the plan depends
+// on the device and the two sizes only).  The launch uses the first kResidentPartials entries of
+// both halves of B.partials and all of B.p2 (cleared here), and ends like
+// launch_pcg_solve_persistent.
+constexpr int kResidentPartials = 4096;
+struct ResidentPlan {
+    int grid = 0;  // 0: not planned
+    int threads = 0;
+    int lanes_per_row = 0;
+    int smem_bytes = 0;
+};
+template <typename T>
+bool plan_pcg_resident(int n_blocks, int64_t nnzb, ResidentPlan& plan);
+template <typename T>
+void launch_pcg_resident(const PcgBuffers<T>& B, const ResidentPlan& plan, cudaStream_t s);
+
 // On the PCG solution du (4 values per block row) and double vectors with 3 per row:
 // out = du . g;  out = max |du|;  x_out = x0 + step * du.
 template <typename T>

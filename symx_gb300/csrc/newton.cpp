@@ -1312,6 +1312,13 @@ SolverReturn solve_t(SolverImpl& I, const NewtonSettings& S, SolveStats& st, int
         B.staged.f64_sums = S.cg_fp64_partial_sums ? 1 : 0;
         B.la = S.cg_lookahead && I.staged.lookahead ? I.la32.p : nullptr;
     }
+    // One-launch PCG: with the matrix in shared memory where it fits (the options of the staged
+    // kernel, residual replacement, FP64 partial sums and look-ahead, keep that one), else the
+    // staged kernel (float), else two launches per iteration.
+    symxg::ResidentPlan resident;
+    const bool staged_options =
+        std::is_same<T, float>::value && (S.cg_residual_replacement > 0 || S.cg_fp64_partial_sums || S.cg_lookahead);
+    const bool use_resident = !staged_options && symxg::plan_pcg_resident<T>(I.n_blocks, I.nnzb, resident);
     T* du = V[0].p;
 
     if (S.linear_solver != LinearSolver::BDPCG) throw std::runtime_error("symx_gb300: only the BDPCG linear solver is implemented");
@@ -1405,8 +1412,8 @@ SolverReturn solve_t(SolverImpl& I, const NewtonSettings& S, SolveStats& st, int
             symxg::launch_pcg_init<T>(B, I.grad.p, s);
             int launched = 0, chunk = 8;
             std::vector<std::pair<cudaEvent_t, cudaEvent_t>> spmv_ev;
-            bool persistent = false;
-            if constexpr (std::is_same<T, float>::value) persistent = B.staged.persistent != 0;
+            bool persistent = use_resident;
+            if constexpr (std::is_same<T, float>::value) persistent |= B.staged.persistent != 0;
             if (persistent) {  // every iteration in one cooperative launch
                 // With residual replacement the launch returns every replace_every iterations;
                 // k_pcg_replace_residual forms the true residual and the next launch continues.
@@ -1421,7 +1428,9 @@ SolverReturn solve_t(SolverImpl& I, const NewtonSettings& S, SolveStats& st, int
                         cudaEventRecord(a, s);
                     }
                     for (int k = 0; k < rounds; ++k) {
-                        if constexpr (std::is_same<T, float>::value) {
+                        if (use_resident) {
+                            symxg::launch_pcg_resident<T>(B, resident, s);
+                        } else if constexpr (std::is_same<T, float>::value) {
                             symxg::launch_pcg_solve_persistent(B, s);
                             if (every > 0) symxg::launch_pcg_replace_residual(B, I.grad.p, s);
                         }
@@ -1434,7 +1443,7 @@ SolverReturn solve_t(SolverImpl& I, const NewtonSettings& S, SolveStats& st, int
                     if (S.time_kernels) {
                         float ms = 0.f;
                         cudaEventElapsedTime(&ms, a, b);
-                        auto& kt = st.kernels["pcg_solve_f32"];
+                        auto& kt = st.kernels[std::string("pcg_solve_") + (sizeof(T) == 4 ? "f32" : "f64")];
                         kt.first += I.h_state->iteration - (round == 0 ? 0 : it_before);
                         kt.second += ms * 1e-3;
                         cudaEventDestroy(a);
@@ -1625,7 +1634,11 @@ AdjointInfo adjoint_pcg_t(SolverImpl& I, const double* rhs, double* lambda, doub
     ck(cudaMemcpyAsync(I.pcg_state.p, &init, sizeof(PcgState), cudaMemcpyHostToDevice, s), "pcg state");
     symxg::launch_pcg_init<T>(B, I.grad.p, s);
     bool done = false;
-    if constexpr (std::is_same<T, float>::value) {
+    symxg::ResidentPlan resident;
+    if (symxg::plan_pcg_resident<T>(I.n_blocks, I.nnzb, resident)) {
+        symxg::launch_pcg_resident<T>(B, resident, s);
+        done = true;
+    } else if constexpr (std::is_same<T, float>::value) {
         if (B.staged.persistent) {
             symxg::launch_pcg_solve_persistent(B, s);
             done = true;
