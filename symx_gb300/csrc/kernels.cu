@@ -362,7 +362,7 @@ __global__ void __launch_bounds__(64) k_project_pd_generic(T* __restrict__ H, in
         }
 }
 
-// Large element matrices (24 x 24 for Hex8): one warp per matrix, parallel cyclic Jacobi in
+// Large FP32 element matrices (30 x 30 for Tet10): one warp per matrix, parallel cyclic Jacobi in
 // the round-robin ("circle method") order: a sweep is N - 1 rounds of N / 2 disjoint index
 // pairs, and one round applies all N / 2 rotations at once, A <- J^T A J with J block diagonal
 // over the pairs.  Written per 2 x 2 block of pairs (k, l) this is B_kl <- R_k^T B_kl R_l, so
@@ -380,20 +380,23 @@ __global__ void __launch_bounds__(64) k_project_pd_generic(T* __restrict__ H, in
 //     are back in their initial order, slot_index() below.
 // Only the upper triangle of A in shared memory is kept up to date.  No two lanes touch the
 // same entry within a round.
-template <typename T, int N>
+template <int N>
 struct ProjPairsCfg {
-    static constexpr int warps = sizeof(T) == 4 ? 8 : 4;
-    // 24 x 24 float: 64 registers, 32 warps per SM; 30 x 30 (Tet10) holds 30 eigenvector
-    // entries per lane and ~90 KB of shared memory per block: two blocks per SM
-    static constexpr int min_blocks = N <= 24 ? 4 : 2;
-    static constexpr int LD = N + 1;  // row stride of A and B (odd: conflict-free columns)
+    static constexpr int warps = 8, max_tile = 512;
+    // 30 eigenvector entries per lane and ~110 KB of shared memory per block: two blocks per SM
+    static constexpr int min_blocks = 2;
+    // row stride of A and B: the four accesses of a round's blocks take 54.6 shared-memory
+    // wavefronts with a stride of 31 and 30.0 with 41 (the least of 31 .. 48); with it and the
+    // sharing of the listed matrices below, 5,940 Hessians went from 1,024 to 631 us
+    static constexpr int LD = N == 30 ? 41 : N + 1;
     static constexpr int VS = (N + 3) / 4 * 4;  // row stride of V in the reconstruction (16-byte rows)
     static constexpr int NP = N / 2, NR = N - 1, NOFF = NP * (NP - 1) / 2, SLOTS = (NOFF + 31) / 32;
-    static constexpr int mat_elems = N * LD > N * VS ? N * LD : N * VS;
+    static constexpr int mat_elems = ((N * LD > N * VS ? N * LD : N * VS) + 3) / 4 * 4;  // rows of V: 16-byte aligned
+    static_assert(VS % 4 == 0 && mat_elems % 4 == 0, "row_dot loads 16 bytes");
     // dynamic shared memory: A and B per warp, (c, s) per warp, the offset table
-    static constexpr size_t off_B = (size_t)warps * mat_elems * sizeof(T);
-    static constexpr size_t off_CS = off_B + (size_t)warps * mat_elems * sizeof(T);
-    static constexpr size_t off_tab = (off_CS + (size_t)warps * NP * 2 * sizeof(T) + 15) / 16 * 16;
+    static constexpr size_t off_B = (size_t)warps * mat_elems * sizeof(float);
+    static constexpr size_t off_CS = off_B + (size_t)warps * mat_elems * sizeof(float);
+    static constexpr size_t off_tab = (off_CS + (size_t)warps * NP * 2 * sizeof(float) + 15) / 16 * 16;
     static constexpr size_t smem_bytes = off_tab + (size_t)NR * SLOTS * 32 * sizeof(uint2);
 };
 
@@ -434,19 +437,8 @@ __device__ __forceinline__ void off_block(int b, int& k, int& l)
     }
 }
 
-template <typename T>
-struct Pair2;
-template <>
-struct Pair2<float> {
-    using type = float2;
-};
-template <>
-struct Pair2<double> {
-    using type = double2;
-};
-
 // sum_{k < N} w[k] * row[k] with 16-byte shared-memory loads (row 16-byte aligned, padded
-// to a multiple of 4 floats / 2 doubles)
+// to a multiple of 4 floats)
 template <int N>
 __device__ __forceinline__ float row_dot(const float (&w)[N], const float* row)
 {
@@ -461,80 +453,67 @@ __device__ __forceinline__ float row_dot(const float (&w)[N], const float* row)
     }
     return acc;
 }
-template <int N>
-__device__ __forceinline__ double row_dot(const double (&w)[N], const double* row)
-{
-    double acc = 0.0;
-#pragma unroll
-    for (int k = 0; k < N; k += 2) {
-        const double2 r = *reinterpret_cast<const double2*>(row + k);
-        acc = fma(w[k], r.x, acc);
-        if (k + 1 < N) acc = fma(w[k + 1 < N ? k + 1 : k], r.y, acc);
-    }
-    return acc;
-}
 
-template <typename T>
-__device__ __forceinline__ T warp_allmax(T v)
+__device__ __forceinline__ float warp_allmax(float v)
 {
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
+    for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
     return v;
 }
 
-// Warp test of one N x N element Hessian A (shared memory, row stride N + 1): true when A is
+// Warp test of one N x N element Hessian A (shared memory, row stride LD): true when A is
 // translation-invariant (max |A t| <= tol max |A|) and Q^T A Q (Q the Helmert basis of the
 // node space orthogonal to (1, ..., 1), (x) I3) has a Cholesky factorization with pivots above
 // 16 M u of its largest diagonal entry.  A is then positive definite in the complement of the
 // translations up to rounding, and the reference's projection would only lift the three
 // translation eigenvalues from 0 to eps, a change below the rounding of A's entries.  B (the
 // same shape) is scratch; every decision is taken by all lanes alike.
-template <typename T, int N>
-__device__ bool pairs_pd_shortcut(const T* __restrict__ A, T* __restrict__ B, int lane)
+template <int N, int LD>
+__device__ bool pairs_pd_shortcut(const float* __restrict__ A, float* __restrict__ B, int lane)
 {
-    constexpr int LD = N + 1, NB = N / 3, M = N - 3;
+    constexpr int NB = N / 3, M = N - 3;
     // rows of A Q (lane i < N: row i): prefix sums over the node blocks; the full sums are
     // the translation residual of the row
-    T amax = T(0), res = T(0);
+    float amax = 0.0f, res = 0.0f;
     if (lane < N) {
-        T acc[3] = {T(0), T(0), T(0)};
+        float acc[3] = {0.0f, 0.0f, 0.0f};
 #pragma unroll
         for (int m = 0; m < NB; ++m)
 #pragma unroll
             for (int e = 0; e < 3; ++e) {
-                const T a = A[lane * LD + 3 * m + e];
+                const float a = A[lane * LD + 3 * m + e];
                 amax = fmax(amax, fabs(a));
-                if (m >= 1) B[lane * LD + 3 * (m - 1) + e] = (acc[e] - T(m) * a) / sqrt(T(m * (m + 1)));
+                if (m >= 1) B[lane * LD + 3 * (m - 1) + e] = (acc[e] - float(m) * a) / sqrt(float(m * (m + 1)));
                 acc[e] += a;
             }
         res = fmax(fabs(acc[0]), fmax(fabs(acc[1]), fabs(acc[2])));
     }
     amax = warp_allmax(amax);
     res = warp_allmax(res);
-    if (!(res <= symxg_dev::DeflationTol<T>::value() * amax)) return false;
+    if (!(res <= symxg_dev::DeflationTol<float>::value() * amax)) return false;
     __syncwarp();
     // columns of Q^T (A Q) (lane c < M: column c), written over rows 0 .. M-1 of the same column
     if (lane < M) {
-        T acc[3] = {T(0), T(0), T(0)};
+        float acc[3] = {0.0f, 0.0f, 0.0f};
 #pragma unroll
         for (int m = 0; m < NB; ++m)
 #pragma unroll
             for (int d = 0; d < 3; ++d) {
-                const T t = B[(3 * m + d) * LD + lane];
-                if (m >= 1) B[(3 * (m - 1) + d) * LD + lane] = (acc[d] - T(m) * t) / sqrt(T(m * (m + 1)));
+                const float t = B[(3 * m + d) * LD + lane];
+                if (m >= 1) B[(3 * (m - 1) + d) * LD + lane] = (acc[d] - float(m) * t) / sqrt(float(m * (m + 1)));
                 acc[d] += t;
             }
     }
     __syncwarp();
     // Cholesky (lower triangle, in place): lane i holds row i
-    const T dmax = warp_allmax(lane < M ? B[lane * LD + lane] : T(0));
-    const T tau = T(16 * M) * symxg_dev::UnitRoundoff<T>::value() * dmax;
+    const float dmax = warp_allmax(lane < M ? B[lane * LD + lane] : 0.0f);
+    const float tau = float(16 * M) * symxg_dev::UnitRoundoff<float>::value() * dmax;
     for (int j = 0; j < M; ++j) {
-        const T d = B[j * LD + j];  // the same value in every lane
+        const float d = B[j * LD + j];  // the same value in every lane
         if (!(d > tau)) return false;
-        const T r = T(1) / sqrt(d);
+        const float r = 1.0f / sqrt(d);
         const bool mine = lane > j && lane < M;
-        const T lij = mine ? B[lane * LD + j] * r : T(0);
+        const float lij = mine ? B[lane * LD + j] * r : 0.0f;
         __syncwarp();
         if (mine) B[lane * LD + j] = lij;
         __syncwarp();
@@ -545,14 +524,13 @@ __device__ bool pairs_pd_shortcut(const T* __restrict__ A, T* __restrict__ B, in
     return true;
 }
 
-template <typename T, int N>
-__global__ void __launch_bounds__(ProjPairsCfg<T, N>::warps * 32, ProjPairsCfg<T, N>::min_blocks)
-    k_project_pd_pairs(T* __restrict__ H, int64_t count, T eps, int mirroring, int* not_converged,
+template <int N>
+__global__ void __launch_bounds__(ProjPairsCfg<N>::warps * 32, ProjPairsCfg<N>::min_blocks)
+    k_project_pd_pairs(float* __restrict__ H, int64_t count, int tile, float eps, int mirroring, int* not_converged,
                        const int64_t* __restrict__ sel)
 {
     static_assert(N % 6 == 0 && N <= 30, "N a multiple of 6 up to 30 (3 x 3 blocks, pairs of indices)");
-    using T2 = typename Pair2<T>::type;
-    using Cfg = ProjPairsCfg<T, N>;
+    using Cfg = ProjPairsCfg<N>;
     constexpr int W = Cfg::warps, LD = Cfg::LD, VS = Cfg::VS;
     constexpr int NP = Cfg::NP, NR = Cfg::NR, NOFF = Cfg::NOFF, SLOTS = Cfg::SLOTS, nb = N / 3;
     // dynamic shared memory (Cfg::smem_bytes): per warp A and a deflated copy B (the
@@ -560,10 +538,12 @@ __global__ void __launch_bounds__(ProjPairsCfg<T, N>::warps * 32, ProjPairsCfg<T
     // lane the 4 x 16-bit entry offsets of an off-diagonal pair block
     extern __shared__ __align__(16) unsigned char pairs_smem[];
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    T* sA = reinterpret_cast<T*>(pairs_smem) + (size_t)w * Cfg::mat_elems;
-    T* sB = reinterpret_cast<T*>(pairs_smem + Cfg::off_B) + (size_t)w * Cfg::mat_elems;
-    T2* sCS = reinterpret_cast<T2*>(pairs_smem + Cfg::off_CS) + (size_t)w * NP;
+    float* sA = reinterpret_cast<float*>(pairs_smem) + (size_t)w * Cfg::mat_elems;
+    float* sB = reinterpret_cast<float*>(pairs_smem + Cfg::off_B) + (size_t)w * Cfg::mat_elems;
+    float2* sCS = reinterpret_cast<float2*>(pairs_smem + Cfg::off_CS) + (size_t)w * NP;
     uint2* sTab = reinterpret_cast<uint2*>(pairs_smem + Cfg::off_tab);  // [NR][SLOTS][32]
+    __shared__ short list[Cfg::max_tile];  // matrices of the tile to decompose
+    __shared__ int n_list;
 
     for (int e = threadIdx.x; e < NR * SLOTS * 32; e += blockDim.x) {
         const int r = e / (SLOTS * 32), j = (e / 32) % SLOTS, ln = e % 32, b = ln + 32 * j;
@@ -584,116 +564,135 @@ __global__ void __launch_bounds__(ProjPairsCfg<T, N>::warps * 32, ProjPairsCfg<T
     for (int j = 0; j < SLOTS; ++j) off_block<NP>(lane + 32 * j < NOFF ? lane + 32 * j : 0, bk[j], bl[j]);
     __syncthreads();
 
-    T* A = sA;
-    T2* CS = sCS;
+    float* A = sA;
+    float2* CS = sCS;
     int nc = 0;
-    constexpr int max_sweeps = 2 * symxg_dev::JacobiTol<T>::max_double_sweeps;
-    for (int64_t item = (int64_t)blockIdx.x * W + w; item < count; item += (int64_t)gridDim.x * W) {
-        T* h = H + (sel ? sel[item] : item) * (int64_t)(N * N);
-        T f = T(0);
+    constexpr int max_sweeps = 2 * symxg_dev::JacobiTol<float>::max_double_sweeps;
+    auto load = [&](const float* h) {
+        float f = 0.0f;
         for (int idx = lane; idx < N * N; idx += 32) {  // block-major storage, read in order
             const int blk = idx / 9, r = idx % 9;
             const int i = (blk / nb) * 3 + r / 3, j = (blk % nb) * 3 + r % 3;
-            const T v = h[idx];
+            const float v = h[idx];
             A[i * LD + j] = v;
             f += v * v;
         }
         __syncwarp();
-        if (pairs_pd_shortcut<T, N>(A, sB, lane)) continue;  // H stays as it is
-        T v[N];
-#pragma unroll
-        for (int s = 0; s < N; ++s) v[s] = lane == slot_index<N>(s) ? T(1) : T(0);
-        // every lane takes the same decisions below: sums are reduced, then lane 0's broadcast
-        f = (T)__shfl_sync(0xffffffffu, warp_sum(f), 0);
-        __syncwarp();
-        int sweep = 0;
-        for (; sweep < max_sweeps; ++sweep) {
-            T off = T(0);
-            for (int idx = lane; idx < N * N; idx += 32) {
-                const int i = idx / N, j = idx % N;
-                if (i < j) off += A[i * LD + j] * A[i * LD + j];
-            }
-            off = T(2) * (T)__shfl_sync(0xffffffffu, warp_sum(off), 0);
-            if (!(off > symxg_dev::JacobiTol<T>::rel2() * f)) break;
-#pragma unroll 1
-            for (int r = 0; r < NR; ++r) {
-                if (lane < NP) {
-                    int p, q;
-                    rr_pair<N>(r, lane, p, q);
-                    const int pq = p < q ? p * LD + q : q * LD + p;
-                    const T app = A[p * LD + p], aqq = A[q * LD + q], apq = A[pq];
-                    const T t = symxg_dev::jacobi_t(app, aqq, apq);
-                    const T c = symxg_dev::inv_hypot1(t);
-                    A[p * LD + p] = app - t * apq;
-                    A[q * LD + q] = aqq + t * apq;
-                    A[pq] = T(0);
-                    T2 cs;
-                    cs.x = c;
-                    cs.y = t * c;
-                    CS[lane] = cs;
-                }
-                __syncwarp();
-#pragma unroll
-                for (int j = 0; j < SLOTS; ++j) {
-                    if ((j + 1) * 32 <= NOFF || lane + 32 * j < NOFF) {
-                        const uint2 e = sTab[(r * SLOTS + j) * 32 + lane];
-                        const T2 rk = CS[bk[j]], rl = CS[bl[j]];
-                        const unsigned e00 = e.x & 0xffffu, e01 = e.x >> 16, e10 = e.y & 0xffffu, e11 = e.y >> 16;
-                        const T b00 = A[e00], b01 = A[e01], b10 = A[e10], b11 = A[e11];
-                        const T r00 = rk.x * b00 - rk.y * b10, r01 = rk.x * b01 - rk.y * b11;  // rows of pair k
-                        const T r10 = rk.y * b00 + rk.x * b10, r11 = rk.y * b01 + rk.x * b11;
-                        A[e00] = rl.x * r00 - rl.y * r01;  // columns of pair l
-                        A[e01] = rl.y * r00 + rl.x * r01;
-                        A[e10] = rl.x * r10 - rl.y * r11;
-                        A[e11] = rl.y * r10 + rl.x * r11;
-                    }
-                }
-#pragma unroll
-                for (int k = 0; k < NP; ++k) {  // eigenvector columns: pair k in slots (2k, 2k + 1)
-                    const T2 cs = CS[k];
-                    const T vp = v[2 * k], vq = v[2 * k + 1];
-                    v[2 * k] = cs.x * vp - cs.y * vq;
-                    v[2 * k + 1] = cs.y * vp + cs.x * vq;
-                }
-                // next round's slot order: new[2k] = old[2k + 2], new[N - 2] = old[N - 1],
-                // new[3] = old[0], new[2k + 1] = old[2k - 1] (k >= 2), slot 1 fixed
-                const T v0 = v[0];
-#pragma unroll
-                for (int k = 0; k < NP - 1; ++k) v[2 * k] = v[2 * k + 2];
-                v[N - 2] = v[N - 1];
-#pragma unroll
-                for (int k = NP - 1; k >= 2; --k) v[2 * k + 1] = v[2 * k - 1];
-                v[3] = v0;
-                __syncwarp();
-            }
-        }
-        if (sweep == max_sweeps) nc = 1;
-        T lam = T(0);
-        bool mine = false;
-        if (lane < N) {
-            lam = A[lane * LD + lane];
-            if (lam < eps) {
-                mine = true;
-                lam = mirroring ? -lam : eps;
-            }
-        }
-        const bool changed = __any_sync(0xffffffffu, mine);
-        if (changed) {
-            __syncwarp();  // eigenvalues read before V overwrites A
-            // rows of V with stride VS (a multiple of 4) for 16-byte row reads
-            if (lane < N) {
-#pragma unroll
-                for (int s = 0; s < N; ++s) A[lane * VS + s] = v[s];
-            }
-#pragma unroll
-            for (int s = 0; s < N; ++s) v[s] *= __shfl_sync(0xffffffffu, lam, slot_index<N>(s));  // V diag(lambda)
+        return f;
+    };
+    // a block tests a tile of matrices, then its warps share the listed ones evenly
+    for (int64_t base = (int64_t)blockIdx.x * tile; base < count; base += (int64_t)gridDim.x * tile) {
+        const int n = (int)(count - base < tile ? count - base : tile);
+        auto at = [&](int i) { return H + (sel ? sel[base + i] : base + i) * (int64_t)(N * N); };
+        if (threadIdx.x == 0) n_list = 0;
+        __syncthreads();
+        for (int i = w; i < n; i += W) {
+            load(at(i));
+            // positive definite ones stay as they are
+            if (!pairs_pd_shortcut<N, LD>(A, sB, lane) && lane == 0) list[atomicAdd(&n_list, 1)] = (short)i;
             __syncwarp();
-            if (lane < N) {
-                const int i = lane, bi = (i / 3) * nb, ri = (i % 3) * 3;
-                for (int j = 0; j < N; ++j) h[(bi + j / 3) * 9 + ri + j % 3] = row_dot<N>(v, A + j * VS);
-            }
         }
-        __syncwarp();  // the next matrix reuses this warp's shared memory
+        __syncthreads();
+        const int pending = n_list;
+        for (int item = w; item < pending; item += W) {
+            float* h = at(list[item]);
+            float f = load(h);
+            float v[N];
+#pragma unroll
+            for (int s = 0; s < N; ++s) v[s] = lane == slot_index<N>(s) ? 1.0f : 0.0f;
+            // every lane takes the same decisions below: sums are reduced, then lane 0's broadcast
+            f = __shfl_sync(0xffffffffu, warp_sum(f), 0);
+            __syncwarp();
+            int sweep = 0;
+            for (; sweep < max_sweeps; ++sweep) {
+                float off = 0.0f;
+                for (int idx = lane; idx < N * N; idx += 32) {
+                    const int i = idx / N, j = idx % N;
+                    if (i < j) off += A[i * LD + j] * A[i * LD + j];
+                }
+                off = 2.0f * __shfl_sync(0xffffffffu, warp_sum(off), 0);
+                if (!(off > symxg_dev::JacobiTol<float>::rel2() * f)) break;
+#pragma unroll 1
+                for (int r = 0; r < NR; ++r) {
+                    if (lane < NP) {
+                        int p, q;
+                        rr_pair<N>(r, lane, p, q);
+                        const int pq = p < q ? p * LD + q : q * LD + p;
+                        const float app = A[p * LD + p], aqq = A[q * LD + q], apq = A[pq];
+                        const float t = symxg_dev::jacobi_t(app, aqq, apq);
+                        const float c = symxg_dev::inv_hypot1(t);
+                        A[p * LD + p] = app - t * apq;
+                        A[q * LD + q] = aqq + t * apq;
+                        A[pq] = 0.0f;
+                        float2 cs;
+                        cs.x = c;
+                        cs.y = t * c;
+                        CS[lane] = cs;
+                    }
+                    __syncwarp();
+#pragma unroll
+                    for (int j = 0; j < SLOTS; ++j) {
+                        if ((j + 1) * 32 <= NOFF || lane + 32 * j < NOFF) {
+                            const uint2 e = sTab[(r * SLOTS + j) * 32 + lane];
+                            const float2 rk = CS[bk[j]], rl = CS[bl[j]];
+                            const unsigned e00 = e.x & 0xffffu, e01 = e.x >> 16, e10 = e.y & 0xffffu, e11 = e.y >> 16;
+                            const float b00 = A[e00], b01 = A[e01], b10 = A[e10], b11 = A[e11];
+                            const float r00 = rk.x * b00 - rk.y * b10, r01 = rk.x * b01 - rk.y * b11;  // rows of pair k
+                            const float r10 = rk.y * b00 + rk.x * b10, r11 = rk.y * b01 + rk.x * b11;
+                            A[e00] = rl.x * r00 - rl.y * r01;  // columns of pair l
+                            A[e01] = rl.y * r00 + rl.x * r01;
+                            A[e10] = rl.x * r10 - rl.y * r11;
+                            A[e11] = rl.y * r10 + rl.x * r11;
+                        }
+                    }
+#pragma unroll
+                    for (int k = 0; k < NP; ++k) {  // eigenvector columns: pair k in slots (2k, 2k + 1)
+                        const float2 cs = CS[k];
+                        const float vp = v[2 * k], vq = v[2 * k + 1];
+                        v[2 * k] = cs.x * vp - cs.y * vq;
+                        v[2 * k + 1] = cs.y * vp + cs.x * vq;
+                    }
+                    // next round's slot order: new[2k] = old[2k + 2], new[N - 2] = old[N - 1],
+                    // new[3] = old[0], new[2k + 1] = old[2k - 1] (k >= 2), slot 1 fixed
+                    const float v0 = v[0];
+#pragma unroll
+                    for (int k = 0; k < NP - 1; ++k) v[2 * k] = v[2 * k + 2];
+                    v[N - 2] = v[N - 1];
+#pragma unroll
+                    for (int k = NP - 1; k >= 2; --k) v[2 * k + 1] = v[2 * k - 1];
+                    v[3] = v0;
+                    __syncwarp();
+                }
+            }
+            if (sweep == max_sweeps) nc = 1;
+            float lam = 0.0f;
+            bool mine = false;
+            if (lane < N) {
+                lam = A[lane * LD + lane];
+                if (lam < eps) {
+                    mine = true;
+                    lam = mirroring ? -lam : eps;
+                }
+            }
+            const bool changed = __any_sync(0xffffffffu, mine);
+            if (changed) {
+                __syncwarp();  // eigenvalues read before V overwrites A
+                // rows of V with stride VS (a multiple of 4) for 16-byte row reads
+                if (lane < N) {
+#pragma unroll
+                    for (int s = 0; s < N; ++s) A[lane * VS + s] = v[s];
+                }
+#pragma unroll
+                for (int s = 0; s < N; ++s) v[s] *= __shfl_sync(0xffffffffu, lam, slot_index<N>(s));  // V diag(lambda)
+                __syncwarp();
+                if (lane < N) {
+                    const int i = lane, bi = (i / 3) * nb, ri = (i % 3) * 3;
+                    for (int j = 0; j < N; ++j) h[(bi + j / 3) * 9 + ri + j % 3] = row_dot<N>(v, A + j * VS);
+                }
+            }
+            __syncwarp();  // the next matrix reuses this warp's shared memory
+        }
+        __syncthreads();
     }
     if (nc) *not_converged = 1;
 }
@@ -2779,13 +2778,13 @@ void launch_dot_mixed(const T* a, const double* b, int64_t n, double* partials, 
     check_launch("dot");
 }
 
-// Warp-per-matrix projection (k_project_pd_pairs) of N x N matrices, N = 18, 24 or 30: a
+// Warp-per-matrix projection (k_project_pd_pairs) of 30 x 30 matrices in FP32: a
 // persistent grid of the resident blocks, dynamic shared memory set up once per device.
-template <typename T, int N>
-void launch_project_pd_pairs(T* H, int64_t count, T eps, bool mirroring, int* not_converged, const int64_t* sel,
+template <int N>
+void launch_project_pd_pairs(float* H, int64_t count, float eps, bool mirroring, int* not_converged, const int64_t* sel,
                              cudaStream_t s)
 {
-    using Cfg = ProjPairsCfg<T, N>;
+    using Cfg = ProjPairsCfg<N>;
     constexpr int threads = Cfg::warps * 32;
     static std::mutex m;
     static std::map<int, bool> configured;
@@ -2794,7 +2793,7 @@ void launch_project_pd_pairs(T* H, int64_t count, T eps, bool mirroring, int* no
     {
         std::lock_guard<std::mutex> lock(m);
         if (!configured[dev]) {
-            const cudaError_t e = cudaFuncSetAttribute(k_project_pd_pairs<T, N>,
+            const cudaError_t e = cudaFuncSetAttribute(k_project_pd_pairs<N>,
                                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg::smem_bytes);
             if (e != cudaSuccess)
                 throw std::runtime_error(std::string("symx_gb300: projection shared memory: ") + cudaGetErrorString(e));
@@ -2803,11 +2802,13 @@ void launch_project_pd_pairs(T* H, int64_t count, T eps, bool mirroring, int* no
     }
     int per_sm = 0, sms = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_project_pd_pairs<T, N>, threads, Cfg::smem_bytes);
-    const unsigned grid = (unsigned)std::max(1, sms * std::max(1, per_sm));
-    const unsigned need = blocks_for(count, Cfg::warps);
-    k_project_pd_pairs<T, N><<<need < grid ? need : grid, threads, Cfg::smem_bytes, s>>>(H, count, eps, mirroring,
-                                                                                        not_converged, sel);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_project_pd_pairs<N>, threads, Cfg::smem_bytes);
+    const int64_t resident = std::max(1, sms * std::max(1, per_sm));
+    // small counts: a matrix per warp on as many blocks as that takes; large ones: equal tiles
+    const int tile = (int)std::min<int64_t>(Cfg::max_tile, std::max<int64_t>(Cfg::warps, (count + resident - 1) / resident));
+    const unsigned grid = (unsigned)std::min<int64_t>(resident, (count + tile - 1) / tile);
+    k_project_pd_pairs<N><<<grid, threads, Cfg::smem_bytes, s>>>(H, count, tile, eps, mirroring, not_converged, sel);
+    check_launch("project_pd_pairs");
 }
 
 template <typename T>
@@ -2815,6 +2816,14 @@ void launch_project_pd(T* H, int N, int64_t count, T eps, bool mirroring, int* n
                        ProjectionScratch scratch, const int64_t* sel)
 {
     if (count <= 0) return;
+    if (launch_project_pd_warp<T>(H, N, count, eps, mirroring, not_converged, sel, s)) return;
+    // 30 x 30 in float keeps the order of rotations of k_project_pd_pairs (see k_project_pd_warp)
+    if constexpr (std::is_same<T, float>::value) {
+        if (N == 30) {
+            launch_project_pd_pairs<30>(H, count, eps, mirroring, not_converged, sel, s);
+            return;
+        }
+    }
     if (N == 12 && scratch.fallback && scratch.n_fallback) {
         const bool split = scratch.pending && scratch.n_pending;
         const cudaError_t e = cudaMemsetAsync(scratch.n_fallback, 0, sizeof(unsigned long long), s);
@@ -2849,9 +2858,6 @@ void launch_project_pd(T* H, int N, int64_t count, T eps, bool mirroring, int* n
         case 6: k_project_pd_unrolled<T, 6><<<blocks_for(count, 128), 128, 0, s>>>(H, count, eps, mirroring, not_converged, sel); break;
         case 9: k_project_pd_unrolled<T, 9><<<blocks_for(count, 128), 128, 0, s>>>(H, count, eps, mirroring, not_converged, sel); break;
         case 12: k_project_pd_unrolled<T, 12><<<blocks_for(count, 128), 128, 0, s>>>(H, count, eps, mirroring, not_converged, sel); break;
-        case 18: launch_project_pd_pairs<T, 18>(H, count, eps, mirroring, not_converged, sel, s); break;
-        case 24: launch_project_pd_pairs<T, 24>(H, count, eps, mirroring, not_converged, sel, s); break;
-        case 30: launch_project_pd_pairs<T, 30>(H, count, eps, mirroring, not_converged, sel, s); break;
         default:
             if (N > 30 || N % 3 != 0) throw std::runtime_error("symx_gb300: projection supports N = 3k <= 30");
             k_project_pd_generic<T><<<blocks_for(count, 64), 64, 0, s>>>(H, N, count, eps, mirroring, not_converged, sel);

@@ -85,6 +85,12 @@ template <typename T>
 void launch_project_pd(T* H, int N, int64_t count, T eps, bool mirroring, int* not_converged, cudaStream_t s,
                        ProjectionScratch scratch = ProjectionScratch{}, const int64_t* sel = nullptr);
 
+// The forms of launch_project_pd with a group of lanes per matrix (project_warp.cu): N = 18 and 24,
+// in double also 12 and 30; false for another N, without a launch.
+template <typename T>
+bool launch_project_pd_warp(T* H, int N, int64_t count, T eps, bool mirroring, int* not_converged, const int64_t* sel,
+                            cudaStream_t s);
+
 // 12 x 12 projection whose arithmetic is FP64-accurate for float or double storage: the
 // sorting pass, then for the listed matrices an FP32 cyclic Jacobi refined by one FP64
 // Ogita-Aishima step, the clamping applied as an FP64 correction and rounded once into H

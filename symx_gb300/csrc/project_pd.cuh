@@ -467,10 +467,9 @@ SYMXG_DEVICE void load_upper(const T* __restrict__ H, T (&a)[N * (N + 1) / 2], T
         }
 }
 
-// b = Q^T H Q (upper triangle) of a translation-invariant H; returns false (b unset) when the
-// translation residual max |H t| exceeds tol * max |H|.
+// b = Q^T H Q (upper triangle) from the upper triangle a of H.
 template <typename T, int NB>
-SYMXG_DEVICE bool deflate_translations(const T* __restrict__ H, T (&b)[(3 * NB - 3) * (3 * NB - 2) / 2])
+SYMXG_DEVICE void deflate_upper(const T (&a)[3 * NB * (3 * NB + 1) / 2], T (&b)[(3 * NB - 3) * (3 * NB - 2) / 2])
 {
     constexpr int N = 3 * NB;
     constexpr int M = N - 3;
@@ -478,21 +477,6 @@ SYMXG_DEVICE bool deflate_translations(const T* __restrict__ H, T (&b)[(3 * NB -
     c[0] = T(0);
 #pragma unroll
     for (int m = 1; m < NB; ++m) c[m] = T(1) / sqrt(T(m * (m + 1)));
-    T a[N * (N + 1) / 2];
-    T hmax = T(0);
-    load_upper<T, N>(H, a, hmax);
-    // translation residual: (H t_e) at row (i, d), up to the factor 1/sqrt(NB)
-    T res = T(0);
-#pragma unroll
-    for (int i = 0; i < N; ++i)
-#pragma unroll
-        for (int e = 0; e < 3; ++e) {
-            T r = T(0);
-#pragma unroll
-            for (int jn = 0; jn < NB; ++jn) r += a[tri<N>(i, 3 * jn + e)];
-            res = fmax(res, fabs(r));
-        }
-    if (!(res <= DeflationTol<T>::value() * hmax)) return false;
     // b = Q^T H Q (upper triangle), row (m, d) of b = row 3 (m - 1) + d
 #pragma unroll
     for (int p = 0; p < M; ++p)
@@ -509,6 +493,30 @@ SYMXG_DEVICE bool deflate_translations(const T* __restrict__ H, T (&b)[(3 * NB -
             }
             b[tri<M>(p, q)] = s;
         }
+}
+
+// b = Q^T H Q (upper triangle) of a translation-invariant H; returns false (b unset) when the
+// translation residual max |H t| exceeds tol * max |H|.
+template <typename T, int NB>
+SYMXG_DEVICE bool deflate_translations(const T* __restrict__ H, T (&b)[(3 * NB - 3) * (3 * NB - 2) / 2])
+{
+    constexpr int N = 3 * NB;
+    T a[N * (N + 1) / 2];
+    T hmax = T(0);
+    load_upper<T, N>(H, a, hmax);
+    // translation residual: (H t_e) at row (i, d), up to the factor 1/sqrt(NB)
+    T res = T(0);
+#pragma unroll
+    for (int i = 0; i < N; ++i)
+#pragma unroll
+        for (int e = 0; e < 3; ++e) {
+            T r = T(0);
+#pragma unroll
+            for (int jn = 0; jn < NB; ++jn) r += a[tri<N>(i, 3 * jn + e)];
+            res = fmax(res, fabs(r));
+        }
+    if (!(res <= DeflationTol<T>::value() * hmax)) return false;
+    deflate_upper<T, NB>(a, b);
     return true;
 }
 
