@@ -214,7 +214,8 @@ int64_t symxg_wait_poll_limit(void);
  * (a,b) at offset (a*k+b)*9, row-major inside), in place.  not_converged: device int set
  * to 1 if a Jacobi sweep cap was hit.  Replaces project_to_PD_inplace
  * (symx/src/solver/second_order/project_to_PD.cpp:12-81).  n = 3..12 run one matrix per
- * thread in registers, n = 18, 24, 30 one matrix per warp in shared memory.  n = 15, 21, 27
+ * thread in registers (n = 12 in f64: ten lanes per matrix), n = 18, 24, 30 one matrix per warp
+ * in shared memory.  n = 15, 21, 27
  * run one matrix per thread with the matrix and its eigenvectors in local memory: the first
  * such call makes the driver reserve local memory for every thread the device can hold
  * (several GB in f64), which the context keeps until it is destroyed. */
@@ -222,6 +223,12 @@ int symxg_project_pd_f32(float* matrices, int32_t n, int64_t count, float eps, i
                          int32_t* not_converged, void* stream);
 int symxg_project_pd_f64(double* matrices, int32_t n, int64_t count, double eps, int32_t mirroring,
                          int32_t* not_converged, void* stream);
+/* The same for row-major matrices, n = 12, 18, 24 or 30, count < 2^31 - 2.  work: 2 + count device
+ * ints, the first two zero on entry; work[0] is not_converged. */
+int symxg_project_pd_rows_f32(float* matrices, int32_t n, int64_t count, float eps, int32_t mirroring,
+                              int32_t* work, void* stream);
+int symxg_project_pd_rows_f64(double* matrices, int32_t n, int64_t count, double eps, int32_t mirroring,
+                              int32_t* work, void* stream);
 /* y = A x for a 3x3-block CSR matrix: row_ptr (n_blocks+1), cols (nnzb) and values stored
  * component-major, i.e. component m (row-major inside the 3x3 block) of block k at
  * vals[m * vals_stride + k], vals_stride >= nnzb (the layout the solver's PCG uses).

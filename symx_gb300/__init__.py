@@ -193,24 +193,32 @@ class ElasticSolver:
 
 
 def project_pd(H, eps=1e-10, mirroring=False, stream=None):
-    """Project a CUDA torch tensor of shape (count, n, n) in place (block-major storage is
-    handled here: the tensor is row-major, converted around the kernel call)."""
+    """Project a CUDA torch tensor of shape (count, n, n) in place.  Contiguous matrices are
+    projected where they lie when the library takes them row-major (n = 12, 18, 24, 30);
+    others go through a block-major copy."""
     import torch
 
-    count, n, _ = H.shape
+    count, n, m = H.shape
+    L = load()
+    current = torch.cuda.current_stream(H.device).cuda_stream
+    s = C.c_void_p(stream if stream is not None else current)
+    f = {torch.float32: "f32", torch.float64: "f64"}
+    # tensors that autograd watches and other streams keep the copy, whose write-back torch orders
+    if (H.dtype in f and n == m and n in (12, 18, 24, 30) and H.is_contiguous() and type(H) is torch.Tensor
+            and not (H.requires_grad or H.is_inference() or H.is_neg()) and (stream is None or stream == current)):
+        work = torch.empty(2 + count, dtype=torch.int32, device=H.device)
+        work[:2].zero_()
+        run = getattr(L, "symxg_project_pd_rows_" + f[H.dtype])
+        check(run(C.c_void_p(H.data_ptr()), n, count, eps, int(mirroring), C.c_void_p(work.data_ptr()), s))
+        torch.autograd.graph.increment_version(H)
+        return bool(work[0].item())
     k = n // 3
     bm = H.reshape(count, k, 3, k, 3).permute(0, 1, 3, 2, 4).contiguous()
-    flag = torch.zeros(1, dtype=torch.int32, device=H.device)
-    L = load()
-    s = C.c_void_p(stream if stream is not None else torch.cuda.current_stream(H.device).cuda_stream)
-    if H.dtype == torch.float32:
-        check(L.symxg_project_pd_f32(C.c_void_p(bm.data_ptr()), n, count, C.c_float(eps), int(mirroring),
-                                     C.c_void_p(flag.data_ptr()), s))
-    elif H.dtype == torch.float64:
-        check(L.symxg_project_pd_f64(C.c_void_p(bm.data_ptr()), n, count, eps, int(mirroring),
-                                     C.c_void_p(flag.data_ptr()), s))
-    else:
+    if H.dtype not in f:
         raise TypeError("float32 or float64 expected")
+    flag = torch.zeros(1, dtype=torch.int32, device=H.device)
+    run = getattr(L, "symxg_project_pd_" + f[H.dtype])
+    check(run(C.c_void_p(bm.data_ptr()), n, count, eps, int(mirroring), C.c_void_p(flag.data_ptr()), s))
     H.copy_(bm.permute(0, 1, 3, 2, 4).reshape(count, n, n))
     return bool(flag.item())
 

@@ -26,7 +26,7 @@ EXPORTS = [
     "symxg_destroy", "symxg_set_settings", "symxg_set_state", "symxg_get_positions", "symxg_solve",
     "symxg_upload", "symxg_solve_device", "symxg_download", "symxg_evaluate", "symxg_evaluate_energy",
     "symxg_assembled_hessian", "symxg_element_outputs", "symxg_op_counts", "symxg_project_pd_f32",
-    "symxg_project_pd_f64", "symxg_bcsr_spmv_f32", "symxg_bcsr_spmv_f64", "symxg_launch_count",
+    "symxg_project_pd_f64", "symxg_project_pd_rows_f32", "symxg_project_pd_rows_f64", "symxg_bcsr_spmv_f32", "symxg_bcsr_spmv_f64", "symxg_launch_count",
     "symxg_bcsr_pcg_f32", "symxg_bcsr_pcg_f64", "symxg_bcsr_pcg_f32_noalloc", "symxg_adjoint",
     "symxg_generate_cuboid_mesh",
     "symxg_rollout_forward", "symxg_rollout_backward", "symxg_set_wait_poll_limit", "symxg_wait_poll_limit",
@@ -156,6 +156,8 @@ def load(path: str | None = None):
         "symxg_generate_cuboid_mesh": ([I32, P, P, C.POINTER(I64), C.POINTER(I64), C.POINTER(I32), P, P], C.c_int),
         "symxg_project_pd_f32": ([P, I32, I64, C.c_float, I32, P, P], C.c_int),
         "symxg_project_pd_f64": ([P, I32, I64, D, I32, P, P], C.c_int),
+        "symxg_project_pd_rows_f32": ([P, I32, I64, C.c_float, I32, P, P], C.c_int),
+        "symxg_project_pd_rows_f64": ([P, I32, I64, D, I32, P, P], C.c_int),
         "symxg_bcsr_spmv_f32": ([I32, P, P, P, I64, P, P, P], C.c_int),
         "symxg_bcsr_spmv_f64": ([I32, P, P, P, I64, P, P, P], C.c_int),
         "symxg_bcsr_pcg_f32": ([I32, P, P, P, I64, P, P, D, D, I32, C.POINTER(PcgInfo), P], C.c_int),

@@ -98,6 +98,19 @@ static int project_impl(T* m, int32_t n, int64_t count, T eps, int32_t mirroring
 }
 
 template <typename T>
+static int project_rows_impl(T* m, int32_t n, int64_t count, T eps, int32_t mirroring, int32_t* work, void* stream)
+{
+    return guarded([&] {
+        if (n != 12 && n != 18 && n != 24 && n != 30) throw std::invalid_argument("n must be 12, 18, 24 or 30");
+        if (count < 0 || count > INT32_MAX - 2) throw std::invalid_argument("count out of range");
+        if (count == 0) return SYMXG_OK;
+        if (!m || !work) throw std::invalid_argument("null device pointer");
+        symxg::launch_project_pd_rows<T>(m, n, count, eps, mirroring != 0, work, (cudaStream_t)stream);
+        return SYMXG_OK;
+    });
+}
+
+template <typename T>
 static int spmv_impl(int32_t nb, const int32_t* rp, const int32_t* cols, const T* vals, int64_t vs, const T* x, T* y,
                      void* stream)
 {
@@ -583,6 +596,14 @@ int symxg_project_pd_f32(float* m, int32_t n, int64_t count, float eps, int32_t 
 int symxg_project_pd_f64(double* m, int32_t n, int64_t count, double eps, int32_t mirroring, int32_t* nc, void* stream)
 {
     return project_impl<double>(m, n, count, eps, mirroring, nc, stream);
+}
+int symxg_project_pd_rows_f32(float* m, int32_t n, int64_t count, float eps, int32_t mirroring, int32_t* work, void* stream)
+{
+    return project_rows_impl<float>(m, n, count, eps, mirroring, work, stream);
+}
+int symxg_project_pd_rows_f64(double* m, int32_t n, int64_t count, double eps, int32_t mirroring, int32_t* work, void* stream)
+{
+    return project_rows_impl<double>(m, n, count, eps, mirroring, work, stream);
 }
 
 int symxg_bcsr_spmv_f32(int32_t nb, const int32_t* rp, const int32_t* cols, const float* vals, int64_t vs, const float* x,

@@ -239,6 +239,19 @@ __global__ void __launch_bounds__(128) k_project_pd_listed(T* __restrict__ H, co
     if (nc) *not_converged = 1;
 }
 
+// Full projection of the row-major matrices listed by k_project_pd_rows12.
+template <int N>
+__global__ void __launch_bounds__(128) k_project_pd_listed_rows(float* __restrict__ H, const int* __restrict__ list,
+                                                                const int* n_list, float eps, int mirroring,
+                                                                int* not_converged)
+{
+    const int n = *n_list;
+    int nc = 0;
+    for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += (int64_t)gridDim.x * blockDim.x)
+        symxg_dev::project_pd_inplace_packed<N, true>(H + (int64_t)list[k] * (N * N), eps, mirroring != 0, &nc);
+    if (nc) *not_converged = 1;
+}
+
 // FP64-accurate projection (symxg_dev::project_pd_refined: FP32 Jacobi, one FP64 refinement
 // step, clamping applied as an FP64 correction) of the matrices k_project_pd_sort listed,
 // grid-stride over the list.  Deflate: the `pending` list (translation-invariant matrices),
@@ -524,7 +537,7 @@ __device__ bool pairs_pd_shortcut(const float* __restrict__ A, float* __restrict
     return true;
 }
 
-template <int N>
+template <int N, bool Rows>
 __global__ void __launch_bounds__(ProjPairsCfg<N>::warps * 32, ProjPairsCfg<N>::min_blocks)
     k_project_pd_pairs(float* __restrict__ H, int64_t count, int tile, float eps, int mirroring, int* not_converged,
                        const int64_t* __restrict__ sel)
@@ -570,9 +583,9 @@ __global__ void __launch_bounds__(ProjPairsCfg<N>::warps * 32, ProjPairsCfg<N>::
     constexpr int max_sweeps = 2 * symxg_dev::JacobiTol<float>::max_double_sweeps;
     auto load = [&](const float* h) {
         float f = 0.0f;
-        for (int idx = lane; idx < N * N; idx += 32) {  // block-major storage, read in order
+        for (int idx = lane; idx < N * N; idx += 32) {  // read in storage order
             const int blk = idx / 9, r = idx % 9;
-            const int i = (blk / nb) * 3 + r / 3, j = (blk % nb) * 3 + r % 3;
+            const int i = Rows ? idx / N : (blk / nb) * 3 + r / 3, j = Rows ? idx % N : (blk % nb) * 3 + r % 3;
             const float v = h[idx];
             A[i * LD + j] = v;
             f += v * v;
@@ -687,7 +700,8 @@ __global__ void __launch_bounds__(ProjPairsCfg<N>::warps * 32, ProjPairsCfg<N>::
                 __syncwarp();
                 if (lane < N) {
                     const int i = lane, bi = (i / 3) * nb, ri = (i % 3) * 3;
-                    for (int j = 0; j < N; ++j) h[(bi + j / 3) * 9 + ri + j % 3] = row_dot<N>(v, A + j * VS);
+                    for (int j = 0; j < N; ++j)
+                        h[Rows ? i * N + j : (bi + j / 3) * 9 + ri + j % 3] = row_dot<N>(v, A + j * VS);
                 }
             }
             __syncwarp();  // the next matrix reuses this warp's shared memory
@@ -2780,7 +2794,7 @@ void launch_dot_mixed(const T* a, const double* b, int64_t n, double* partials, 
 
 // Warp-per-matrix projection (k_project_pd_pairs) of 30 x 30 matrices in FP32: a
 // persistent grid of the resident blocks, dynamic shared memory set up once per device.
-template <int N>
+template <int N, bool Rows>
 void launch_project_pd_pairs(float* H, int64_t count, float eps, bool mirroring, int* not_converged, const int64_t* sel,
                              cudaStream_t s)
 {
@@ -2793,7 +2807,7 @@ void launch_project_pd_pairs(float* H, int64_t count, float eps, bool mirroring,
     {
         std::lock_guard<std::mutex> lock(m);
         if (!configured[dev]) {
-            const cudaError_t e = cudaFuncSetAttribute(k_project_pd_pairs<N>,
+            const cudaError_t e = cudaFuncSetAttribute(k_project_pd_pairs<N, Rows>,
                                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg::smem_bytes);
             if (e != cudaSuccess)
                 throw std::runtime_error(std::string("symx_gb300: projection shared memory: ") + cudaGetErrorString(e));
@@ -2802,12 +2816,12 @@ void launch_project_pd_pairs(float* H, int64_t count, float eps, bool mirroring,
     }
     int per_sm = 0, sms = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_project_pd_pairs<N>, threads, Cfg::smem_bytes);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_project_pd_pairs<N, Rows>, threads, Cfg::smem_bytes);
     const int64_t resident = std::max(1, sms * std::max(1, per_sm));
     // small counts: a matrix per warp on as many blocks as that takes; large ones: equal tiles
     const int tile = (int)std::min<int64_t>(Cfg::max_tile, std::max<int64_t>(Cfg::warps, (count + resident - 1) / resident));
     const unsigned grid = (unsigned)std::min<int64_t>(resident, (count + tile - 1) / tile);
-    k_project_pd_pairs<N><<<grid, threads, Cfg::smem_bytes, s>>>(H, count, tile, eps, mirroring, not_converged, sel);
+    k_project_pd_pairs<N, Rows><<<grid, threads, Cfg::smem_bytes, s>>>(H, count, tile, eps, mirroring, not_converged, sel);
     check_launch("project_pd_pairs");
 }
 
@@ -2816,11 +2830,11 @@ void launch_project_pd(T* H, int N, int64_t count, T eps, bool mirroring, int* n
                        ProjectionScratch scratch, const int64_t* sel)
 {
     if (count <= 0) return;
-    if (launch_project_pd_warp<T>(H, N, count, eps, mirroring, not_converged, sel, s)) return;
+    if (launch_project_pd_warp<T, false>(H, N, count, eps, mirroring, not_converged, sel, s)) return;
     // 30 x 30 in float keeps the order of rotations of k_project_pd_pairs (see k_project_pd_warp)
     if constexpr (std::is_same<T, float>::value) {
         if (N == 30) {
-            launch_project_pd_pairs<30>(H, count, eps, mirroring, not_converged, sel, s);
+            launch_project_pd_pairs<30, false>(H, count, eps, mirroring, not_converged, sel, s);
             return;
         }
     }
@@ -2863,6 +2877,27 @@ void launch_project_pd(T* H, int N, int64_t count, T eps, bool mirroring, int* n
             k_project_pd_generic<T><<<blocks_for(count, 64), 64, 0, s>>>(H, N, count, eps, mirroring, not_converged, sel);
     }
     check_launch("project_pd");
+}
+
+template <typename T>
+void launch_project_pd_rows(T* H, int N, int64_t count, T eps, bool mirroring, int* work, cudaStream_t s)
+{
+    if (count <= 0) return;
+    if (launch_project_pd_warp<T, true>(H, N, count, eps, mirroring, work, nullptr, s)) return;
+    if constexpr (std::is_same<T, float>::value) {
+        if (N == 30) {
+            launch_project_pd_pairs<30, true>(H, count, eps, mirroring, work, nullptr, s);
+            return;
+        }
+        if (N == 12) {
+            launch_project_pd_rows12(H, count, eps, mirroring, work, s);
+            const unsigned grid = std::min(resident_grid(k_project_pd_listed_rows<12>, 128), blocks_for(count, 128));
+            k_project_pd_listed_rows<12><<<grid, 128, 0, s>>>(H, work + 2, work + 1, eps, mirroring, work);
+            check_launch("project_pd_listed_rows");
+            return;
+        }
+    }
+    throw std::invalid_argument("symx_gb300: row-major matrices need N = 12, 18, 24 or 30");
 }
 
 template <typename T>
@@ -3193,6 +3228,7 @@ void launch_convert_to_double(int64_t n, const T* x, double* y, cudaStream_t s)
     template void launch_dot_mixed<T>(const T*, const double*, int64_t, double*, unsigned*, double*, cudaStream_t);  \
     template void launch_project_pd_refined12<T>(T*, int64_t, double, bool, int*, cudaStream_t, ProjectionScratch,    \
                                                  const int64_t*);                                                     \
+    template void launch_project_pd_rows<T>(T*, int, int64_t, T, bool, int*, cudaStream_t);                            \
     template void launch_project_pd<T>(T*, int, int64_t, T, bool, int*, cudaStream_t, ProjectionScratch,               \
                                        const int64_t*);                                                                 \
     template void launch_assemble_blocks<T>(int64_t, const int64_t*, const int32_t*, const T*, T*, int64_t, cudaStream_t); \

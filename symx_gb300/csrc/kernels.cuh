@@ -85,11 +85,19 @@ template <typename T>
 void launch_project_pd(T* H, int N, int64_t count, T eps, bool mirroring, int* not_converged, cudaStream_t s,
                        ProjectionScratch scratch = ProjectionScratch{}, const int64_t* sel = nullptr);
 
-// The forms of launch_project_pd with a group of lanes per matrix (project_warp.cu): N = 18 and 24,
-// in double also 12 and 30; false for another N, without a launch.
+// The same for row-major matrices, N = 12, 18, 24 or 30.  work: 2 + count ints, the first two zero on
+// entry; work[0] is not_converged.
 template <typename T>
+void launch_project_pd_rows(T* H, int N, int64_t count, T eps, bool mirroring, int* work, cudaStream_t s);
+
+// The forms with a group of lanes per matrix (project_warp.cu): N = 18 and 24, in double also 12 and
+// 30; false for another N, without a launch.
+template <typename T, bool Rows>
 bool launch_project_pd_warp(T* H, int N, int64_t count, T eps, bool mirroring, int* not_converged, const int64_t* sel,
                             cudaStream_t s);
+// Row-major 12 x 12 in float: all but the matrices that are not translation-invariant, which are listed
+// (work[1] of them from work + 2 on).
+void launch_project_pd_rows12(float* H, int64_t count, float eps, bool mirroring, int* work, cudaStream_t s);
 
 // 12 x 12 projection whose arithmetic is FP64-accurate for float or double storage: the
 // sorting pass, then for the listed matrices an FP32 cyclic Jacobi refined by one FP64

@@ -30,6 +30,13 @@ SYMXG_DEVICE constexpr int bm_index(int i, int j)
     return (((i / 3) * (N / 3) + (j / 3)) * 3 + (i % 3)) * 3 + (j % 3);
 }
 
+// Entry (i, j) in block-major or, with Rows, row-major storage.
+template <int N, bool Rows>
+SYMXG_DEVICE constexpr int h_index(int i, int j)
+{
+    return Rows ? i * N + j : bm_index<N>(i, j);
+}
+
 template <int N>
 SYMXG_DEVICE constexpr int tri(int i, int j)
 {
@@ -217,7 +224,7 @@ SYMXG_DEVICE void jacobi_step_packed(float (&a)[N * (N + 1) / 2], float2 (&vv)[(
     }
 }
 
-template <int N>
+template <int N, bool Rows = false>
 SYMXG_DEVICE int project_pd_inplace_packed(float* __restrict__ H, float eps, bool mirroring, int* not_converged)
 {
     constexpr int NT = N * (N + 1) / 2;
@@ -226,7 +233,7 @@ SYMXG_DEVICE int project_pd_inplace_packed(float* __restrict__ H, float eps, boo
 #pragma unroll
     for (int i = 0; i < N; ++i)
 #pragma unroll
-        for (int j = i; j < N; ++j) a[tri<N>(i, j)] = H[bm_index<N>(i, j)];
+        for (int j = i; j < N; ++j) a[tri<N>(i, j)] = H[h_index<N, Rows>(i, j)];
 #pragma unroll
     for (int kp = 0; kp < N / 2; ++kp)
 #pragma unroll
@@ -274,11 +281,11 @@ SYMXG_DEVICE int project_pd_inplace_packed(float* __restrict__ H, float eps, boo
                 const float w = lam[k] * ((j & 1) ? vj.y : vj.x);
                 acc = __ffma2_rn(vv[ip * N + k], make_float2(w, w), acc);
             }
-            H[bm_index<N>(2 * ip, j)] = acc.x;
-            H[bm_index<N>(j, 2 * ip)] = acc.x;
+            H[h_index<N, Rows>(2 * ip, j)] = acc.x;
+            H[h_index<N, Rows>(j, 2 * ip)] = acc.x;
             if (j >= 2 * ip + 1) {
-                H[bm_index<N>(2 * ip + 1, j)] = acc.y;
-                H[bm_index<N>(j, 2 * ip + 1)] = acc.y;
+                H[h_index<N, Rows>(2 * ip + 1, j)] = acc.y;
+                H[h_index<N, Rows>(j, 2 * ip + 1)] = acc.y;
             }
         }
     return 1;
@@ -432,10 +439,10 @@ SYMXG_DEVICE bool positive_definite_by_cholesky(const T (&b)[M * (M + 1) / 2])
     return true;
 }
 
-// Upper triangle of the symmetric block-major matrix H into a, and max |entry| into hmax.  A
+// Upper triangle of the symmetric matrix H (block-major; row-major with Rows) into a, and max |entry| into hmax.  A
 // 16-byte aligned float matrix is read with 16-byte loads in storage order (N * N / 4 of
 // them instead of N (N + 1) / 2 scalar loads).
-template <typename T, int N>
+template <typename T, int N, bool Rows = false>
 SYMXG_DEVICE void load_upper(const T* __restrict__ H, T (&a)[N * (N + 1) / 2], T& hmax)
 {
 #ifdef __CUDA_ARCH__
@@ -449,7 +456,8 @@ SYMXG_DEVICE void load_upper(const T* __restrict__ H, T (&a)[N * (N + 1) / 2], T
 #pragma unroll
                 for (int t = 0; t < 4; ++t) {
                     const int idx = 4 * q + t, blk = idx / 9, r = idx % 9;
-                    const int i = (blk / (N / 3)) * 3 + r / 3, j = (blk % (N / 3)) * 3 + r % 3;
+                    const int i = Rows ? idx / N : (blk / (N / 3)) * 3 + r / 3;
+                    const int j = Rows ? idx % N : (blk % (N / 3)) * 3 + r % 3;
                     if (i <= j) a[tri<N>(i, j)] = vv[t];
                     hmax = fmax(hmax, fabs(vv[t]));
                 }
@@ -462,7 +470,7 @@ SYMXG_DEVICE void load_upper(const T* __restrict__ H, T (&a)[N * (N + 1) / 2], T
     for (int i = 0; i < N; ++i)
 #pragma unroll
         for (int j = i; j < N; ++j) {
-            a[tri<N>(i, j)] = H[bm_index<N>(i, j)];
+            a[tri<N>(i, j)] = H[h_index<N, Rows>(i, j)];
             hmax = fmax(hmax, fabs(a[tri<N>(i, j)]));
         }
 }
@@ -497,13 +505,13 @@ SYMXG_DEVICE void deflate_upper(const T (&a)[3 * NB * (3 * NB + 1) / 2], T (&b)[
 
 // b = Q^T H Q (upper triangle) of a translation-invariant H; returns false (b unset) when the
 // translation residual max |H t| exceeds tol * max |H|.
-template <typename T, int NB>
+template <typename T, int NB, bool Rows = false>
 SYMXG_DEVICE bool deflate_translations(const T* __restrict__ H, T (&b)[(3 * NB - 3) * (3 * NB - 2) / 2])
 {
     constexpr int N = 3 * NB;
     T a[N * (N + 1) / 2];
     T hmax = T(0);
-    load_upper<T, N>(H, a, hmax);
+    load_upper<T, N, Rows>(H, a, hmax);
     // translation residual: (H t_e) at row (i, d), up to the factor 1/sqrt(NB)
     T res = T(0);
 #pragma unroll
@@ -522,7 +530,7 @@ SYMXG_DEVICE bool deflate_translations(const T* __restrict__ H, T (&b)[(3 * NB -
 
 // Eigen-decomposition of b = Q^T H Q, clamping, and H = Q W Q^T + lam_t / NB (1 1^T (x) I3).
 // Returns 1 when H changed.
-template <typename T, int NB>
+template <typename T, int NB, bool Rows = false>
 SYMXG_DEVICE int project_deflated_finish(T* __restrict__ H, T (&b)[(3 * NB - 3) * (3 * NB - 2) / 2], T eps,
                                          bool mirroring, int* not_converged)
 {
@@ -584,8 +592,8 @@ SYMXG_DEVICE int project_deflated_finish(T* __restrict__ H, T (&b)[(3 * NB - 3) 
                 }
                 s += helmert<T, NB>(c, in, m) * t;
             }
-            H[bm_index<N>(i, j)] = s;
-            H[bm_index<N>(j, i)] = s;
+            H[h_index<N, Rows>(i, j)] = s;
+            H[h_index<N, Rows>(j, i)] = s;
         }
     return 1;
 }

@@ -1,6 +1,7 @@
 // Projection of element Hessians to positive definite by a group of lanes per matrix:
 // k_project_pd_warp (18 x 18 and 24 x 24 in float and double, 30 x 30 in double, one warp per matrix)
-// and k_project_pd_tile12 (12 x 12 in double, three matrices per warp).
+// and k_project_pd_tile12 (12 x 12 in double, three matrices per warp); and row-major 12 x 12 in
+// float by a thread per matrix (k_project_pd_rows12).
 //
 // Reference: project_to_PD_inplace (symx/src/solver/second_order/project_to_PD.cpp:12-81), applied
 // per element by ElementHessians.cpp:48-67.
@@ -229,7 +230,8 @@ struct Jacobi {
         __device__ __forceinline__ bool operator()(const T*, int, int, T a) const { return fabsf((float)a) > tol; }
     };
     // Sweeps until no entry above the diagonal is `open` in a group whose `work` is set; false in a
-    // group that reached the cap.  Entries below negligible (under the rounding of max |H|) are dropped
+    // group that reached the cap.  A group without open entries sits the others' sweeps out: its result
+    // does not depend on the matrices that share its warp.  Entries below negligible (under the rounding of max |H|) are dropped
     // instead of rotated: between equal eigenvalues such an entry would turn its pair by 45 degrees in
     // every sweep and mix what the other rotations have separated.
     template <typename Open>
@@ -248,8 +250,8 @@ struct Jacobi {
             if (sweep == max_sweeps) return !open;
 #pragma unroll 1
             for (int r = 0; r < M / 2; ++r) {
-                round<0>(A, CS, v, gl, member, negligible);
-                round<1>(A, CS, v, gl, member, negligible);
+                round<0>(A, CS, v, gl, member && open, negligible);
+                round<1>(A, CS, v, gl, member && open, negligible);
             }
         }
     }
@@ -314,7 +316,7 @@ struct GroupMem {
 // The matrix h times `scale` into g.a (row-major), amax = max |entry| of it, and g.b = Q^T (scale h) Q
 // (M x M).  Returns whether it is translation-invariant: max |H t| <= tol max |H|.  In double, scale
 // is the power of two that brings amax into [1, 2), so the float stages cannot overflow.
-template <typename T, int N, int L>
+template <typename T, int N, int L, bool Rows>
 __device__ __forceinline__ bool load_and_deflate(const T* __restrict__ h, const GroupMem<T, N>& g, int gl, bool member,
                                                  bool work, float& amax, T& scale)
 {
@@ -322,10 +324,10 @@ __device__ __forceinline__ bool load_and_deflate(const T* __restrict__ h, const 
     const Helmert<T, NB> hm;
     T hmax = T(0);
     if (work)
-        for (int idx = gl; idx < N * N; idx += L) {  // block-major storage, read in order
+        for (int idx = gl; idx < N * N; idx += L) {  // read in storage order
             const int blk = idx / 9, r = idx % 9;
             const T v = h[idx];
-            g.a[((blk / NB) * 3 + r / 3) * LD + (blk % NB) * 3 + r % 3] = v;
+            g.a[Rows ? (idx / N) * LD + idx % N : ((blk / NB) * 3 + r / 3) * LD + (blk % NB) * 3 + r % 3] = v;
             hmax = fmax(hmax, fabs(v));
         }
     scale = T(1);
@@ -412,7 +414,7 @@ constexpr int kMaxSweepsFloat = 16, kMaxSweepsDouble = 20;
 
 // Steps 3 to 5 for a loaded matrix: B = g.b when deflated, else g.a.  Returns false in a group that
 // reached a sweep cap.
-template <typename T, int N, int L, bool Deflate>
+template <typename T, int N, int L, bool Deflate, bool Rows>
 __device__ __forceinline__ bool decompose_and_correct(T* __restrict__ h, const GroupMem<T, N>& g, int gl, bool member,
                                                       bool work, float amax, T scale, T eps, bool mirroring)
 {
@@ -576,7 +578,7 @@ __device__ __forceinline__ bool decompose_and_correct(T* __restrict__ h, const G
     if constexpr (!Deflate) {
         if (work && changed && gl < M)
 #pragma unroll
-            for (int j = 0; j < M; ++j) h[((gl / 3) * NB + j / 3) * 9 + (gl % 3) * 3 + j % 3] += w[j] * unscale;
+            for (int j = 0; j < M; ++j) h[Rows ? gl * N + j : ((gl / 3) * NB + j / 3) * 9 + (gl % 3) * 3 + j % 3] += w[j] * unscale;
     } else {
         // Q w Q^T by suffix sums over the nodes: columns of the own row, then rows of the own columns;
         // the translations' eigenvalues 0 -> eps (0 when mirroring)
@@ -607,11 +609,11 @@ __device__ __forceinline__ bool decompose_and_correct(T* __restrict__ h, const G
                 for (int d = 0; d < 3; ++d) {
                     const T lift = c % 3 == d ? lam_t / T(NB) : T(0);
                     T tail = T(0);
-                    T* const hc = h + (c / 3) * 9 + d * 3 + c % 3;
+                    T* const hc = h + (Rows ? d * N + c : (c / 3) * 9 + d * 3 + c % 3);
 #pragma unroll
                     for (int m = NB - 1; m >= 1; --m) {
                         const T t = hm.c[m] * W[(3 * (m - 1) + d) * LD + c];
-                        hc[m * NB * 9] += (tail - T(m) * t + lift) * unscale;
+                        hc[m * 3 * N] += (tail - T(m) * t + lift) * unscale;
                         tail += t;
                     }
                     hc[0] += (tail + lift) * unscale;
@@ -643,7 +645,7 @@ struct WarpCfg {
     static constexpr size_t smem = warps * GroupMem<T, N>::bytes;
 };
 
-template <typename T, int N>
+template <typename T, int N, bool Rows>
 __global__ void __launch_bounds__(WarpCfg<T, N>::warps * 32, WarpCfg<T, N>::min_blocks)
     k_project_pd_warp(T* __restrict__ H, int64_t count, int tile, T eps, int mirroring, int* not_converged,
                       const int64_t* __restrict__ sel)
@@ -663,7 +665,7 @@ __global__ void __launch_bounds__(WarpCfg<T, N>::warps * 32, WarpCfg<T, N>::min_
         if (threadIdx.x == 0) n_list = 0;
         __syncthreads();
         for (int i = w; i < n; i += W) {
-            const bool invariant = load_and_deflate<T, N, 32>(at(i), g, lane, true, true, amax, scale);
+            const bool invariant = load_and_deflate<T, N, 32, Rows>(at(i), g, lane, true, true, amax, scale);
             bool done = false;
             if (invariant)
                 done = positive_definite<T, N - 3, kStride<N>>(g.b, reinterpret_cast<float*>(sizeof(T) == 8 ? g.s : g.a), lane);
@@ -675,11 +677,11 @@ __global__ void __launch_bounds__(WarpCfg<T, N>::warps * 32, WarpCfg<T, N>::min_
         for (int k = w; k < pending; k += W) {
             const int i = list[k];
             T* h = at(i < 0 ? -1 - i : i);
-            load_and_deflate<T, N, 32>(h, g, lane, true, true, amax, scale);
+            load_and_deflate<T, N, 32, Rows>(h, g, lane, true, true, amax, scale);
             if (i >= 0)
-                ok = decompose_and_correct<T, N, 32, true>(h, g, lane, true, true, amax, scale, eps, mirroring != 0) && ok;
+                ok = decompose_and_correct<T, N, 32, true, Rows>(h, g, lane, true, true, amax, scale, eps, mirroring != 0) && ok;
             else
-                ok = decompose_and_correct<T, N, 32, false>(h, g, lane, true, true, amax, scale, eps, mirroring != 0) && ok;
+                ok = decompose_and_correct<T, N, 32, false, Rows>(h, g, lane, true, true, amax, scale, eps, mirroring != 0) && ok;
         }
         __syncthreads();
     }
@@ -696,6 +698,7 @@ constexpr int kTileThreads = 128;
 
 // 0: positive definite in the complement of the translations, 1: to be decomposed there, 2: not
 // translation-invariant.
+template <bool Rows>
 __device__ __forceinline__ int classify12(const double* __restrict__ h)
 {
     constexpr int N = 12, NB = 4, M = 9;
@@ -707,7 +710,7 @@ __device__ __forceinline__ int classify12(const double* __restrict__ h)
         double acc[3] = {0.0, 0.0, 0.0};
 #pragma unroll
         for (int j = 0; j < N; ++j) {
-            const double v = h[symxg_dev::bm_index<N>(i, j)];
+            const double v = h[symxg_dev::h_index<N, Rows>(i, j)];
             if (i <= j) a[symxg_dev::tri<N>(i, j)] = (float)v;
             hmax = fmax(hmax, fabs(v));
             acc[j % 3] += v;
@@ -725,6 +728,7 @@ __device__ __forceinline__ int classify12(const double* __restrict__ h)
     return symxg_dev::positive_definite_by_cholesky<float, M>(b) ? 0 : 1;
 }
 
+template <bool Rows>
 __global__ void __launch_bounds__(kTileThreads, 3)
     k_project_pd_tile12(double* __restrict__ H, int64_t count, int tile, double eps, int mirroring, int* not_converged,
                         const int64_t* __restrict__ sel)
@@ -741,12 +745,12 @@ __global__ void __launch_bounds__(kTileThreads, 3)
         __syncthreads();
         if (tid < tile && base + tid < count) {
             const int64_t m = sel ? sel[base + tid] : base + tid;
-            const int c = classify12(H + m * (N * N));
+            const int c = classify12<Rows>(H + m * (N * N));
             if (c) list[c - 1][atomicAdd(&n_list[c - 1], 1)] = m;
         }
         __syncthreads();
         const int n1 = n_list[0], n2 = n_list[1];
-        const int turn = (w + blockIdx.x) % W;  // the SM's blocks start on different quarters
+        const int turn = (w + (int)((int64_t)blockIdx.x * W / gridDim.x)) % W;  // an SM's blocks start on different quarters
         for (int i0 = turn * 3; i0 < n1; i0 += 3 * W) {
             const int grp = lane / 10, gl = lane % 10;
             const bool member = grp < 3, work = member && i0 + grp < n1;
@@ -754,8 +758,8 @@ __global__ void __launch_bounds__(kTileThreads, 3)
             double* h = H + (work ? list[0][i0 + grp] : 0) * (N * N);
             float amax;
             double scale;
-            load_and_deflate<double, N, 10>(h, g, gl, member, work, amax, scale);
-            ok = decompose_and_correct<double, N, 10, true>(h, g, gl, member, work, amax, scale, eps, mirroring != 0) && ok;
+            load_and_deflate<double, N, 10, Rows>(h, g, gl, member, work, amax, scale);
+            ok = decompose_and_correct<double, N, 10, true, Rows>(h, g, gl, member, work, amax, scale, eps, mirroring != 0) && ok;
         }
         for (int i0 = turn * 2; i0 < n2; i0 += 2 * W) {
             const int grp = lane / 16, gl = lane % 16;
@@ -764,12 +768,54 @@ __global__ void __launch_bounds__(kTileThreads, 3)
             double* h = H + (work ? list[1][i0 + grp] : 0) * (N * N);
             float amax;
             double scale;
-            load_and_deflate<double, N, 16>(h, g, gl, true, work, amax, scale);
-            ok = decompose_and_correct<double, N, 16, false>(h, g, gl, true, work, amax, scale, eps, mirroring != 0) && ok;
+            load_and_deflate<double, N, 16, Rows>(h, g, gl, true, work, amax, scale);
+            ok = decompose_and_correct<double, N, 16, false, Rows>(h, g, gl, true, work, amax, scale, eps, mirroring != 0) && ok;
         }
         __syncthreads();
     }
     if (!ok) *not_converged = 1;
+}
+
+// ---- row-major 12 x 12 in float: tiles of matrices, a thread per matrix
+// A block tests a tile of matrices and lists those to decompose; its warps then share the list, so
+// the decompositions (Jacobi in registers, bound by issue) run in full warps.  The blocks take the
+// matrices in turn: neighbouring elements tend to be indefinite together.  200,003 Hessians of a
+// deformed mesh through project_pd: 591 us with block-major copies around a kernel that tests and
+// decomposes in the same thread (318 us), 314 us with this one on the rows themselves (225 us).
+constexpr int kMaxTile12 = 1024;
+__global__ void __launch_bounds__(kTileThreads, 3)
+    k_project_pd_rows12(float* __restrict__ H, int64_t count, int tile, float eps, int mirroring, int* __restrict__ work)
+{
+    constexpr int N = 12, M = 9, W = kTileThreads / 32;
+    __shared__ short list[kMaxTile12];
+    __shared__ int n_list;
+    const int tid = threadIdx.x;
+    // the blocks of an SM start their lists on different quarters of it
+    const int first = ((tid >> 5) + (int)((int64_t)blockIdx.x * W / gridDim.x)) % W * 32 + (tid & 31);
+    int nc = 0;
+    for (int64_t base = blockIdx.x; base < count; base += (int64_t)gridDim.x * tile) {
+        const int64_t left = (count - base + gridDim.x - 1) / gridDim.x;
+        const int n = (int)(left < tile ? left : tile);
+        if (tid == 0) n_list = 0;
+        __syncthreads();
+        for (int i = tid; i < n; i += kTileThreads) {
+            const int64_t m = base + (int64_t)i * gridDim.x;
+            float b[M * (M + 1) / 2];
+            if (!symxg_dev::deflate_translations<float, N / 3, true>(H + m * (N * N), b))
+                work[2 + atomicAdd(work + 1, 1)] = (int)m;
+            else if (!symxg_dev::positive_definite_by_cholesky<float, M>(b))  // those stay as they are
+                list[atomicAdd(&n_list, 1)] = (short)i;
+        }
+        __syncthreads();
+        for (int k = first; k < n_list; k += kTileThreads) {
+            float* h = H + (base + (int64_t)list[k] * gridDim.x) * (N * N);
+            float b[M * (M + 1) / 2];
+            if (symxg_dev::deflate_translations<float, N / 3, true>(h, b))
+                symxg_dev::project_deflated_finish<float, N / 3, true>(h, b, eps, mirroring != 0, &nc);
+        }
+        __syncthreads();
+    }
+    if (nc) work[0] = 1;
 }
 
 // Dynamic shared memory of `kernel` allowed once per device, and its blocks resident at once.
@@ -800,49 +846,67 @@ void check(const char* what)
         throw std::runtime_error(std::string("symx_gb300: launch of ") + what + " failed: " + cudaGetErrorString(e));
 }
 
-template <typename T, int N>
+// Matrices per tile: the count shared evenly by the resident blocks in as few passes as `most` allows,
+// at least `least`.
+int tile_size(int64_t count, int64_t resident, int least, int most)
+{
+    const int64_t passes = (count + resident * most - 1) / (resident * most);
+    return (int)std::max<int64_t>(least, (count + resident * passes - 1) / (resident * passes));
+}
+
+template <typename T, int N, bool Rows>
 void launch_warp(T* H, int64_t count, T eps, bool mirroring, int* not_converged, const int64_t* sel, cudaStream_t s)
 {
     using Cfg = WarpCfg<T, N>;
-    const int64_t resident = resident_blocks(k_project_pd_warp<T, N>, Cfg::warps * 32, Cfg::smem);
-    // small counts: a matrix per warp on as many blocks as that takes; large ones: equal tiles
-    const int tile = (int)std::min<int64_t>(kMaxTile, std::max<int64_t>(Cfg::warps, (count + resident - 1) / resident));
+    const int64_t resident = resident_blocks(k_project_pd_warp<T, N, Rows>, Cfg::warps * 32, Cfg::smem);
+    const int tile = tile_size(count, resident, Cfg::warps, kMaxTile);
     const int64_t grid = std::min<int64_t>(resident, (count + tile - 1) / tile);
-    k_project_pd_warp<T, N><<<(unsigned)grid, Cfg::warps * 32, Cfg::smem, s>>>(H, count, tile, eps, mirroring, not_converged, sel);
+    k_project_pd_warp<T, N, Rows><<<(unsigned)grid, Cfg::warps * 32, Cfg::smem, s>>>(H, count, tile, eps, mirroring, not_converged,
+                                                                                    sel);
     check("project_pd_warp");
 }
 
-void launch_project_pd_tile12(double* H, int64_t count, double eps, bool mirroring, int* not_converged,
-                              const int64_t* sel, cudaStream_t s)
+template <bool Rows>
+void launch_tile12(double* H, int64_t count, double eps, bool mirroring, int* not_converged, const int64_t* sel, cudaStream_t s)
 {
     const size_t smem = (kTileThreads / 32) * 3 * GroupMem<double, 12>::bytes;
-    const int64_t grid = resident_blocks(k_project_pd_tile12, kTileThreads, smem);
-    // small counts are spread over every block; a full tile fills the sorting pass's threads
-    const int tile = (int)std::min<int64_t>(kTileThreads, std::max<int64_t>(1, (count + grid - 1) / grid));
-    k_project_pd_tile12<<<(unsigned)std::min<int64_t>(grid, (count + tile - 1) / tile), kTileThreads, smem, s>>>(
-        H, count, tile, eps, mirroring, not_converged, sel);
+    const int64_t resident = resident_blocks(k_project_pd_tile12<Rows>, kTileThreads, smem);
+    const int tile = tile_size(count, resident, 1, kTileThreads);
+    const int64_t grid = std::min<int64_t>(resident, (count + tile - 1) / tile);
+    k_project_pd_tile12<Rows><<<(unsigned)grid, kTileThreads, smem, s>>>(H, count, tile, eps, mirroring, not_converged, sel);
     check("project_pd_tile12");
 }
 
 }  // namespace
 
-template <typename T>
+void launch_project_pd_rows12(float* H, int64_t count, float eps, bool mirroring, int* work, cudaStream_t s)
+{
+    const int64_t resident = resident_blocks(k_project_pd_rows12, kTileThreads, 0);
+    const int tile = tile_size(count, resident, 32, kMaxTile12);
+    const int64_t grid = std::min<int64_t>(resident, (count + tile - 1) / tile);
+    k_project_pd_rows12<<<(unsigned)grid, kTileThreads, 0, s>>>(H, count, tile, eps, mirroring, work);
+    check("project_pd_rows12");
+}
+
+template <typename T, bool Rows>
 bool launch_project_pd_warp(T* H, int N, int64_t count, T eps, bool mirroring, int* not_converged, const int64_t* sel,
                             cudaStream_t s)
 {
-    switch (N) {
-        case 18: launch_warp<T, 18>(H, count, eps, mirroring, not_converged, sel, s); return true;
-        case 24: launch_warp<T, 24>(H, count, eps, mirroring, not_converged, sel, s); return true;
-        default: break;
-    }
-    if constexpr (sizeof(T) == 8) {
-        if (N == 12) launch_project_pd_tile12(H, count, eps, mirroring, not_converged, sel, s);
-        if (N == 30) launch_warp<T, 30>(H, count, eps, mirroring, not_converged, sel, s);
-        return N == 12 || N == 30;
-    }
-    return false;
+    if (N == 18) launch_warp<T, 18, Rows>(H, count, eps, mirroring, not_converged, sel, s);
+    else if (N == 24) launch_warp<T, 24, Rows>(H, count, eps, mirroring, not_converged, sel, s);
+    else if constexpr (sizeof(T) == 8) {
+        if (N == 12) launch_tile12<Rows>(H, count, eps, mirroring, not_converged, sel, s);
+        else if (N == 30) launch_warp<T, 30, Rows>(H, count, eps, mirroring, not_converged, sel, s);
+        else return false;
+    } else
+        return false;
+    return true;
 }
-template bool launch_project_pd_warp<float>(float*, int, int64_t, float, bool, int*, const int64_t*, cudaStream_t);
-template bool launch_project_pd_warp<double>(double*, int, int64_t, double, bool, int*, const int64_t*, cudaStream_t);
+#define INSTANTIATE(T, ROWS) \
+    template bool launch_project_pd_warp<T, ROWS>(T*, int, int64_t, T, bool, int*, const int64_t*, cudaStream_t);
+INSTANTIATE(float, false)
+INSTANTIATE(float, true)
+INSTANTIATE(double, false)
+INSTANTIATE(double, true)
 
 }  // namespace symxg

@@ -48,7 +48,8 @@ def _matrices(n, count, seed):
 
 @pytest.mark.parametrize("mirroring", [False, True])
 @pytest.mark.parametrize("n,dtype,count", [(12, "float64", 1), (12, "float64", 7), (12, "float64", 129),
-                                           (12, "float64", 3001), (18, "float32", 33), (18, "float64", 33),
+                                           (12, "float64", 3001), (12, "float32", 1), (12, "float32", 33),
+                                           (12, "float32", 1500), (18, "float32", 33), (18, "float64", 33),
                                            (24, "float32", 9), (24, "float64", 141), (30, "float32", 141),
                                            (30, "float64", 15)])
 def test_projection_matches_eigh(lib, n, dtype, count, mirroring):
@@ -87,3 +88,53 @@ def test_extreme_scales_and_nan(lib):
         keep = np.arange(6) != 2
         ref = _reference(H[keep], 1e-6, False)
         assert np.max(np.abs(got.cpu().numpy()[keep] - ref)) <= TOL["float64"] * np.abs(H[keep]).max()
+
+
+@pytest.mark.parametrize("n,dtype", [(12, "float32"), (12, "float64"), (18, "float32"), (24, "float64"), (30, "float32")])
+def test_contiguous_and_strided_matrices_agree(lib, n, dtype):
+    """Contiguous matrices are projected where they lie, others through a block-major copy: the
+    same operations, so the same bits; views that share the storage see the result."""
+    import torch
+
+    import symx_gb300 as sg
+
+    H = torch.tensor(_matrices(n, 97, seed=5).astype(dtype), device="cuda")
+    rows, wide = H.clone(), torch.zeros(97, n, 2 * n, dtype=H.dtype, device="cuda")
+    wide[:, :, :n] = H
+    sg.project_pd(rows, eps=1e-6)
+    sg.project_pd(wide[:, :, :n], eps=1e-6)
+    assert torch.equal(rows, wide[:, :, :n]) and not torch.equal(rows, H)
+    assert not wide[:, :, n:].any()
+    shifted = torch.zeros(H.numel() + 1, dtype=H.dtype, device="cuda")  # not 16-byte aligned
+    shifted[1:] = H.flatten()
+    sg.project_pd(shifted[1:].view_as(H), eps=1e-6)
+    assert torch.equal(shifted[1:].view_as(H), rows) and shifted[0] == 0
+
+
+def test_autograd_sees_the_projection(lib):
+    import torch
+
+    import symx_gb300 as sg
+
+    H = torch.tensor(_matrices(12, 7, seed=6), device="cuda")
+    version = H._version
+    sg.project_pd(H)
+    assert H._version > version
+    leaf = H.clone().requires_grad_()
+    with pytest.raises(RuntimeError):
+        sg.project_pd(leaf)
+
+
+@pytest.mark.parametrize("dtype,copies", [("float32", 4800), ("float64", 600)])
+def test_more_matrices_than_one_pass_of_tiles(lib, dtype, copies):
+    """Several tiles per block; and each matrix's bits do not depend on those next to it."""
+    import torch
+
+    import symx_gb300 as sg
+
+    H = torch.tensor(_matrices(12, 101, seed=8).astype(dtype), device="cuda")
+    few = H.clone()
+    sg.project_pd(few, eps=1e-6)
+    many = H.repeat(copies, 1, 1)
+    sg.project_pd(many, eps=1e-6)
+    assert torch.equal(many, few.repeat(copies, 1, 1))
