@@ -120,6 +120,7 @@ struct CompiledPotential {
     OpCount ops_eg, ops_h, ops_e;
     DevBuf<int32_t> conn;
     DevBuf<const double*> map_ptrs;
+    std::vector<const double*> host_ptrs;  // what map_ptrs holds
     int n_cache = 0, n_qp = 1;      // hoisted values per element and quadrature point
     int qp_lanes = 1;               // lanes per element of the mixed E+g+H kernel (one per quadrature point)
     bool cache_df = false;          // the cache holds (hi, lo) float pairs (mixed-precision kernels)
@@ -309,23 +310,25 @@ std::string build_source(CompiledPotential& cp, const Expressions& g, const std:
         "(long long n, const int* __restrict__ conn, const double* const* __restrict__ maps, "
         "const double* __restrict__ cache, double* __restrict__ E";
 
-    // precompute kernel
+    // precompute kernel: a thread per element and quadrature point, the points of an element n threads apart
     s << "extern \"C\" __global__ void __launch_bounds__(128) symxg_pre(long long n, const int* __restrict__ conn, "
          "const double* const* __restrict__ maps, double* __restrict__ cache)\n{\n";
-    s << "    const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;\n    if (e >= n) return;\n";
+    s << "    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;\n    if (t >= n * " << NQ
+      << ") return;\n    const long long q = t / n, e = t - q * n;\n    (void)e;\n";
     if (K > 0) {
         s << "    double in[" << NS << "];\n    symxg_gather_pre(e, conn, maps, in);\n";
-        s << "    for (int q = 0; q < " << NQ << "; ++q) {\n" << set_sum("q", pre_symbol);
+        s << "    {\n" << set_sum("q", pre_symbol);
         s << "        double c[" << K << "];\n        symxg_eval_pre(in, nullptr, c);\n";
         s << "        for (int k = 0; k < " << K << "; ++k) cache[((long long)q * " << K << "LL + k) * n + e] = c[k];\n    }\n";
     }
     s << "}\n";
 
-    // E + g + H kernels, H in double or float (FP64 with several quadrature points: one lane
+    // E + g (+ H) kernels, H in double or float (FP64 with several quadrature points: one lane
     // per point, as the mixed kernel below)
     if (qp_parallel) {
-        s << "extern \"C\" __global__ void __launch_bounds__(128) symxg_egh_f64" << sig_common
-          << ", double* __restrict__ G, double* __restrict__ H)\n{\n";
+        for (const bool with_h : {true, false}) {
+        s << "extern \"C\" __global__ void __launch_bounds__(128) " << (with_h ? "symxg_egh_f64" : "symxg_eg_f64") << sig_common
+          << ", double* __restrict__ G" << (with_h ? ", double* __restrict__ H" : "") << ")\n{\n";
         s << "    if (n <= 0) return;\n";
         s << "    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;\n";
         s << "    const int lq = (int)(t % SYMXG_NQ);\n    const bool st = t / SYMXG_NQ < n;\n";
@@ -340,25 +343,31 @@ std::string build_source(CompiledPotential& cp, const Expressions& g, const std:
         s << "        if (st && lq == 0) E[e] = eg[0];\n";
         s << "#pragma unroll\n        for (int i = 0; i < " << NG << "; ++i)\n"
           << "            if (st && lq == i % SYMXG_NQ) G[e * " << NG << "LL + i] = eg[1 + i];\n";
-        s << "        symxg_eval_h_f64_q(in, cq, n, H + e * " << NH << "LL, lq, st);\n    }\n}\n";
+        if (with_h) s << "        symxg_eval_h_f64_q(in, cq, n, H + e * " << NH << "LL, lq, st);\n";
+        s << "    }\n}\n";
+        }
     }
-    for (int prec = 0; prec < 2; ++prec) {
-        if (prec == 0 && qp_parallel) continue;
+    // form 0: H in double, 1: H in float, 2: no H (a gradient alone: with H in the FP64 pipe 0.47 ms for
+    // 196,608 tetrahedra, without it 0.15 ms)
+    for (int prec = 0; prec < 3; ++prec) {
+        if (prec != 1 && qp_parallel) continue;
+        const bool with_h = prec < 2;
         const std::string TH = prec == 0 ? "double" : "float";
-        const std::string kname = prec == 0 ? "symxg_egh_f64" : "symxg_egh_f32";
+        const std::string kname = prec == 0 ? "symxg_egh_f64" : prec == 1 ? "symxg_egh_f32" : "symxg_eg_f64";
         s << "extern \"C\" __global__ void __launch_bounds__(128) " << kname << sig_common
-          << ", double* __restrict__ G, " << TH << "* __restrict__ H)\n{\n";
+          << ", double* __restrict__ G" << (with_h ? ", " + TH + "* __restrict__ H" : "") << ")\n{\n";
         s << "    const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;\n    if (e >= n) return;\n";
         s << "    double in[" << NS << "];\n    symxg_gather(e, conn, maps, in);\n";
         std::ostringstream zw;
         zw << "            E[e] = 0.0;\n            for (int i = 0; i < " << NG << "; ++i) G[e * " << NG
-           << "LL + i] = 0.0;\n"
-           << "            for (int i = 0; i < " << NH << "; ++i) H[e * " << NH << "LL + i] = (" << TH << ")0;\n";
+           << "LL + i] = 0.0;\n";
+        if (with_h) zw << "            for (int i = 0; i < " << NH << "; ++i) H[e * " << NH << "LL + i] = (" << TH << ")0;\n";
         s << cond_check(zw.str());
-        s << "    double eg[" << (NG + 1) << "];\n    " << TH << " h[" << NH << "];\n";
+        s << "    double eg[" << (NG + 1) << "];\n";
+        if (with_h) s << "    " << TH << " h[" << NH << "];\n";
         if (acc) {
             s << "    for (int i = 0; i < " << NG + 1 << "; ++i) eg[i] = 0.0;\n";
-            s << "    for (int i = 0; i < " << NH << "; ++i) h[i] = (" << TH << ")0;\n";
+            if (with_h) s << "    for (int i = 0; i < " << NH << "; ++i) h[i] = (" << TH << ")0;\n";
             s << "    for (int q = 0; q < " << NQ << "; ++q) {\n";
         } else {
             s << "    { const int q = 0; (void)q;\n";
@@ -367,7 +376,7 @@ std::string build_source(CompiledPotential& cp, const Expressions& g, const std:
         s << "        symxg_eval_eg(in, c, eg);\n";
         if (prec == 0) {
             s << "        symxg_eval_h_f64(in, c, h);\n";
-        } else {
+        } else if (prec == 1) {
             s << "        float in32[" << NS << "], c32[" << std::max(1, K) << "];\n";
             s << "        for (int i = 0; i < " << NS << "; ++i) in32[i] = (float)in[i];\n";
             s << "        for (int i = 0; i < " << std::max(1, K) << "; ++i) c32[i] = (float)c[i];\n";
@@ -382,6 +391,10 @@ std::string build_source(CompiledPotential& cp, const Expressions& g, const std:
               << "        for (int i = 0; i < " << NG / 2 << "; ++i) G2[i] = make_double2(eg[1 + 2 * i], eg[2 + 2 * i]);\n"
               << "    } else\n";
         s << "    for (int i = 0; i < " << NG << "; ++i) G[e * " << NG << "LL + i] = eg[1 + i];\n";
+        if (!with_h) {
+            s << "}\n";
+            continue;
+        }
         if (prec == 0 && NH % 2 == 0)
             s << "    if ((reinterpret_cast<unsigned long long>(H) & 15ull) == 0ull) {\n"
               << "        double2* H2 = reinterpret_cast<double2*>(H + e * " << NH << "LL);\n"
@@ -671,26 +684,33 @@ struct SolverImpl {
 
     // The element kernels of the mixed path read the hoisted cache as double-float pairs, the
     // FP64 kernels as doubles: convert in place, or recompute the doubles, when the path changes.
+    void compute_cache(CompiledPotential& cp)
+    {
+        if (cp.n_cache == 0 || cp.n_elements == 0) return;
+        long long n = cp.n_elements;
+        const int32_t* conn = cp.conn.p;
+        const double* const* maps = cp.map_ptrs.p;
+        double* cache = cp.cache.p;
+        void* args[] = {&n, &conn, &maps, &cache};
+        cp.module->launch("symxg_pre", dim3((unsigned)((n * cp.n_qp + 127) / 128)), dim3(128), 0, stream, args);
+        cp.cache_df = false;
+    }
     void ensure_cache(CompiledPotential& cp, bool df)
     {
         if (cp.n_cache == 0 || cp.n_elements == 0 || cp.cache_df == df) return;
-        long long n = cp.n_elements;
         if (df) {
-            long long count = n * cp.n_qp * cp.n_cache;
+            long long count = cp.n_elements * (int64_t)cp.n_qp * cp.n_cache;
             double* c = cp.cache.p;
             void* args[] = {&count, &c};
             cp.module->launch("symxg_cache_to_df", dim3((unsigned)((count + 255) / 256)), dim3(256), 0, stream, args);
+            cp.cache_df = true;
         } else {
-            const int32_t* conn = cp.conn.p;
-            const double* const* maps = cp.map_ptrs.p;
-            double* cache = cp.cache.p;
-            void* args[] = {&n, &conn, &maps, &cache};
-            cp.module->launch("symxg_pre", dim3((unsigned)((n + 127) / 128)), dim3(128), 0, stream, args);
+            compute_cache(cp);
         }
-        cp.cache_df = df;
     }
 
-    // mode: 0 E+g+H in FP64, 1 mixed (E+g double-float, H FP32), 2 E only FP64, 3 E only double-float.
+    // mode: 0 E+g+H in FP64, 1 mixed (E+g double-float, H FP32), 2 E only FP64, 3 E only double-float,
+    // 4 E+g in FP64.
     // In the mixed modes, potentials of one DoF block per element (inertia or gravity, penalty
     // boundary conditions) keep E and g in FP64: their coefficients are large (a 1e8 penalty
     // times the rounding of x in double-float, about 1e-15 m, is a gradient error near 1e-7,
@@ -709,14 +729,17 @@ struct SolverImpl {
             const double* cache = cp.cache.p;
             double* E = E_el.p + cp.e_off;
             const unsigned grid = (unsigned)((n + 127) / 128);
-            if (m >= 2) {
+            double* G = g_el.p + cp.g_off * 3;
+            const unsigned grid_eh = (unsigned)((n * cp.qp_lanes + 127) / 128);  // kernels with a lane per point
+            if (m == 4) {
+                void* args[] = {&n, &conn, &maps, &cache, &E, &G};
+                cp.module->launch("symxg_eg_f64", dim3(grid_eh), dim3(128), 0, stream, args);
+            } else if (m >= 2) {
                 void* args[] = {&n, &conn, &maps, &cache, &E};
                 cp.module->launch(m == 2 ? "symxg_e" : "symxg_e_df", dim3(grid), dim3(128), 0, stream, args);
             } else {
-                double* G = g_el.p + cp.g_off * 3;
                 void* H = m == 0 ? (void*)(H64.p + cp.h_off * 9) : (void*)(H32.p + cp.h_off * 9);
                 void* args[] = {&n, &conn, &maps, &cache, &E, &G, &H};
-                const unsigned grid_eh = (unsigned)((n * cp.qp_lanes + 127) / 128);  // both E+g+H kernels
                 const char* kname = m == 0 ? "symxg_egh_f64" : eg64_h32 ? "symxg_egh_f32" : "symxg_egh_df32";
                 cp.module->launch(kname, dim3(eg64_h32 ? grid : grid_eh), dim3(128), 0, stream, args);
             }
@@ -1090,27 +1113,22 @@ void NewtonsMethod::upload()
             }
             ptrs[k] = ua->dev.p;
         }
-        // arrays are re-read on every upload: the user may change them between solves
-        ck(cudaMemcpyAsync(cp.map_ptrs.p, ptrs.data(), sizeof(double*) * ptrs.size(), cudaMemcpyHostToDevice, I.stream),
-           "upload map pointers");
-        bytes += (int64_t)(sizeof(double*) * ptrs.size());
-        ck(cudaStreamSynchronize(I.stream), "synchronize");
+        // the pointers change only when an array is bound anew
+        if (ptrs != cp.host_ptrs) {
+            cp.host_ptrs = std::move(ptrs);
+            ck(cudaMemcpyAsync(cp.map_ptrs.p, cp.host_ptrs.data(), sizeof(double*) * cp.host_ptrs.size(),
+                               cudaMemcpyHostToDevice, I.stream),
+               "upload map pointers");
+            bytes += (int64_t)(sizeof(double*) * cp.host_ptrs.size());
+        }
     }
+    // arrays are re-read on every upload: the user may change them between solves
     for (auto& a : I.arrays) {
         ck(cudaMemcpyAsync(a.dev.p, a.host, sizeof(double) * a.n, cudaMemcpyHostToDevice, I.stream), "upload data");
         bytes += (int64_t)sizeof(double) * a.n;
     }
     // values that depend only on the uploaded data are computed once here
-    for (auto& cp : I.pots) {
-        if (cp.n_cache == 0 || cp.n_elements == 0) continue;
-        long long n = cp.n_elements;
-        const int32_t* conn = cp.conn.p;
-        const double* const* maps = cp.map_ptrs.p;
-        double* cache = cp.cache.p;
-        void* args[] = {&n, &conn, &maps, &cache};
-        cp.module->launch("symxg_pre", dim3((unsigned)((n + 127) / 128)), dim3(128), 0, I.stream, args);
-        cp.cache_df = false;
-    }
+    for (auto& cp : I.pots) I.compute_cache(cp);
     ck(cudaStreamSynchronize(I.stream), "synchronize");
     h2d_bytes_ = bytes;
 }
@@ -1148,13 +1166,13 @@ double NewtonsMethod::evaluate_energy()
 double NewtonsMethod::evaluate(double* grad_host)
 {
     SolverImpl& I = *impl;
-    I.ensure_precision(Precision::FP64);
-    I.launch_eval(0);
+    I.launch_eval(4);
     symxg::launch_sum(I.E_el.p, I.n_elements_total, I.partials.p, I.tickets.p + 4, I.scalars.p, I.stream);
     symxg::launch_gather_gradient(I.n_blocks, I.gptr.p, I.gcontrib.p, I.g_el.p, I.grad.p, I.stream);
-    I.read_scalars(1);
     if (grad_host)
-        ck(cudaMemcpy(grad_host, I.grad.p, sizeof(double) * I.n_dofs, cudaMemcpyDeviceToHost), "download gradient");
+        ck(cudaMemcpyAsync(grad_host, I.grad.p, sizeof(double) * I.n_dofs, cudaMemcpyDeviceToHost, I.stream),
+           "download gradient");
+    I.read_scalars(1);
     return I.h_scalars[0];
 }
 
