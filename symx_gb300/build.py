@@ -41,7 +41,7 @@ def _headers_mtime() -> float:
     m = 0.0
     for d in (CSRC, INCLUDE):
         for f in os.listdir(d):
-            if f.endswith((".h", ".cuh", ".hpp")) or f == "symx":
+            if f.endswith((".h", ".cuh", ".hpp", ".inl")) or f == "symx":
                 m = max(m, os.path.getmtime(os.path.join(d, f)))
     return m
 

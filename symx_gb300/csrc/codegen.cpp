@@ -63,7 +63,9 @@ struct symxg_df {
     __device__ __forceinline__ void operator+=(const symxg_df& b);
     __device__ __forceinline__ void operator*=(const symxg_df& b);
 };
-__device__ __forceinline__ double symxg_to_double(const symxg_df& a) { return (double)a.hi + (double)a.lo; }
+)"
+#include "df_convert.inl"
+           R"(__device__ __forceinline__ double symxg_to_double(const symxg_df& a) { return (double)a.hi + (double)a.lo; }
 // hoisted values read where they are used: (hi, lo) pairs of the mixed path's cache
 __device__ __forceinline__ symxg_df symxg_ldc_df(const float2* __restrict__ p, long long i)
 {

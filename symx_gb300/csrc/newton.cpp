@@ -408,9 +408,19 @@ std::string build_source(CompiledPotential& cp, const Expressions& g, const std:
         s << "    for (int i = 0; i < " << NH << "; ++i) H[e * " << NH << "LL + i] = h[i];\n}\n";
     }
     // ---- mixed precision: the cache holds (hi, lo) float pairs in place of the doubles
-    s << "extern \"C\" __global__ void __launch_bounds__(256) symxg_cache_to_df(long long count, double* cache)\n{\n"
-         "    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;\n    if (i >= count) return;\n"
-         "    const symxg_df v(cache[i]);\n    reinterpret_cast<float2*>(cache)[i] = make_float2(v.hi, v.lo);\n}\n";
+    // (the formulas as a call: predicated, their FP64 instructions would hold the pipe although off)
+    s << "static __device__ __noinline__ symxg_df symxg_split_f64(double x) { return symxg_df(x); }\n"
+         "extern \"C\" __global__ void __launch_bounds__(256) symxg_cache_to_df(long long count, double* cache)\n{\n"
+         "    const long long i0 = 1024LL * blockIdx.x + 2 * threadIdx.x;  // pairs of values i0 and i0 + 512\n"
+         "    double2 x[2];\n#pragma unroll\n    for (int j = 0; j < 2; ++j) {\n        const long long i = i0 + 512 * j;\n"
+         "        x[j] = i + 1 < count ? *reinterpret_cast<const double2*>(cache + i)\n"
+         "                             : make_double2(i < count ? cache[i] : 0.0, 0.0);\n    }\n"
+         "#pragma unroll\n    for (int j = 0; j < 2; ++j) {\n        const long long i = i0 + 512 * j;\n"
+         "        bool bad = false;\n        symxg_df a = symxg_split(x[j].x, bad), b = symxg_split(x[j].y, bad);\n"
+         "        if (bad) { a = symxg_split_f64(x[j].x); b = symxg_split_f64(x[j].y); }\n"
+         "        float2* p = reinterpret_cast<float2*>(cache) + i;\n"
+         "        if (i + 1 < count) *reinterpret_cast<float4*>(p) = make_float4(a.hi, a.lo, b.hi, b.lo);\n"
+         "        else if (i < count) *p = make_float2(a.hi, a.lo);\n    }\n}\n";
     auto set_sum_df = [&](const std::string& q) {
         std::ostringstream t;
         if (sum.n_iterations == 0 || !sum_used(main_symbol)) return t.str();
@@ -431,13 +441,22 @@ std::string build_source(CompiledPotential& cp, const Expressions& g, const std:
             t << "        c[0] = symxg_df(0.0); c32[0] = 0.0f;\n";
         return t.str();
     };
+    auto gathered = [&](int i) {  // a symbol that the kernels read from the bound data
+        return main_symbol[i] && !(sum.n_iterations > 0 && i >= sum.first_symbol && i < sum.first_symbol + sum.stride);
+    };
     auto head_df = [&]() {
         std::ostringstream t;
         t << "    const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;\n    if (e >= n) return;\n";
         t << "    const float2* __restrict__ cache = reinterpret_cast<const float2*>(cache_raw);\n";
         t << "    double in[" << NS << "];\n    symxg_gather(e, conn, maps, in);\n";
         t << "    symxg_df ind[" << NS << "]; float in32[" << NS << "];\n";
-        t << "    for (int i = 0; i < " << NS << "; ++i) { ind[i] = symxg_df(in[i]); in32[i] = ind[i].hi; }\n";
+        t << "    { bool bad = false;\n";
+        for (int i = 0; i < NS; ++i)
+            if (gathered(i)) t << "    ind[" << i << "] = symxg_split(in[" << i << "], bad);\n";
+        t << "    if (bad) {\n";
+        for (int i = 0; i < NS; ++i)
+            if (gathered(i)) t << "    ind[" << i << "] = symxg_df(in[" << i << "]);\n";
+        t << "    } }\n    for (int i = 0; i < " << NS << "; ++i) in32[i] = ind[i].hi;\n";
         return t.str();
     };
     auto cond_check_df = [&](const std::string& zero_writes) {
@@ -491,14 +510,17 @@ std::string build_source(CompiledPotential& cp, const Expressions& g, const std:
         s << set_sum_df("q");
         s << "        const float2* __restrict__ cq = cache + (long long)q * " << K << "LL * n + e;\n";
         s << "        symxg_eval_eg_dfl(ind, cq, n, eg);\n        symxg_eval_h_f32l(in32, cq, n, h);\n    }\n";
-        s << "    E[e] = symxg_to_double(eg[0]);\n";
+        s << "    double out[" << NG + 1 << "];\n    bool bad = false;\n"
+          << "    for (int i = 0; i < " << NG + 1 << "; ++i) out[i] = symxg_join(eg[i], bad);\n"
+          << "    if (bad) for (int i = 0; i < " << NG + 1 << "; ++i) out[i] = symxg_to_double(eg[i]);\n";
+        s << "    E[e] = out[0];\n";
         // 16-byte stores where the rows allow it (one element's outputs are contiguous)
         if (NG % 2 == 0)
             s << "    if ((reinterpret_cast<unsigned long long>(G) & 15ull) == 0ull) {\n"
               << "        double2* G2 = reinterpret_cast<double2*>(G + e * " << NG << "LL);\n"
-              << "        for (int i = 0; i < " << NG / 2 << "; ++i) G2[i] = make_double2(symxg_to_double(eg[1 + 2 * i]), "
-              << "symxg_to_double(eg[2 + 2 * i]));\n    } else\n";
-        s << "    for (int i = 0; i < " << NG << "; ++i) G[e * " << NG << "LL + i] = symxg_to_double(eg[1 + i]);\n";
+              << "        for (int i = 0; i < " << NG / 2 << "; ++i) G2[i] = make_double2(out[1 + 2 * i], out[2 + 2 * i]);\n"
+              << "    } else\n";
+        s << "    for (int i = 0; i < " << NG << "; ++i) G[e * " << NG << "LL + i] = out[1 + i];\n";
         if (NH % 4 == 0)
             s << "    if ((reinterpret_cast<unsigned long long>(H) & 15ull) == 0ull) {\n"
               << "        float4* H4 = reinterpret_cast<float4*>(H + e * " << NH << "LL);\n"
@@ -702,7 +724,7 @@ struct SolverImpl {
             long long count = cp.n_elements * (int64_t)cp.n_qp * cp.n_cache;
             double* c = cp.cache.p;
             void* args[] = {&count, &c};
-            cp.module->launch("symxg_cache_to_df", dim3((unsigned)((count + 255) / 256)), dim3(256), 0, stream, args);
+            cp.module->launch("symxg_cache_to_df", dim3((unsigned)((count + 1023) / 1024)), dim3(256), 0, stream, args);
             cp.cache_df = true;
         } else {
             compute_cache(cp);
