@@ -150,7 +150,7 @@ __global__ void __launch_bounds__(128) k_project_pd_unrolled(T* __restrict__ H, 
     int nc = 0;
     T* h = H + m * (N * N);
     // Tet4-sized matrices of translation-invariant energies: 9 x 9 decomposition (the
-    // scratch-free form of k_project_pd_deflated + k_project_pd_listed).
+    // scratch-free form of k_project_pd_sort and the listed kernels).
     if constexpr (N == 12) {
         if (symxg_dev::project_pd_deflated<T, N / 3>(h, eps, mirroring != 0, &nc) >= 0) {
             if (nc) *not_converged = 1;
@@ -161,24 +161,6 @@ __global__ void __launch_bounds__(128) k_project_pd_unrolled(T* __restrict__ H, 
         symxg_dev::project_pd_inplace_packed<N>(h, eps, mirroring != 0, &nc);
     else
         symxg_dev::project_pd_inplace<T, N>(h, eps, mirroring != 0, &nc);
-    if (nc) *not_converged = 1;
-}
-
-// Translation-deflated projection (project_pd_deflated) of every matrix whose translation
-// residual is rounding noise; the others are left unchanged and their indices appended to
-// `fallback` (count in *n_fallback, zeroed before the launch) for k_project_pd_listed.
-template <typename T, int N>
-__global__ void __launch_bounds__(128) k_project_pd_deflated(T* __restrict__ H, int64_t count, T eps, int mirroring,
-                                                             int* not_converged, int64_t* __restrict__ fallback,
-                                                             unsigned long long* n_fallback,
-                                                             const int64_t* __restrict__ sel)
-{
-    const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= count) return;
-    const int64_t m = sel ? sel[k] : k;
-    int nc = 0;
-    if (symxg_dev::project_pd_deflated<T, N / 3>(H + m * (N * N), eps, mirroring != 0, &nc) < 0)
-        fallback[atomicAdd(n_fallback, 1ull)] = m;
     if (nc) *not_converged = 1;
 }
 
@@ -221,7 +203,7 @@ __global__ void __launch_bounds__(128) k_project_pd_deflated_listed(T* __restric
     if (nc) *not_converged = 1;
 }
 
-// Full projection of the matrices listed by k_project_pd_deflated (grid-stride over the list).
+// Full projection of the matrices k_project_pd_sort listed in `fallback` (grid-stride over the list).
 template <typename T, int N>
 __global__ void __launch_bounds__(128) k_project_pd_listed(T* __restrict__ H, const int64_t* __restrict__ list,
                                                            const unsigned long long* n_list, T eps, int mirroring,
@@ -2873,47 +2855,40 @@ void launch_project_pd(T* H, int N, int64_t count, T eps, bool mirroring, int* n
 {
     if (count <= 0) return;
     if (launch_project_pd_warp<T, false>(H, N, count, eps, mirroring, not_converged, sel, s)) return;
-    // 30 x 30 in float keeps the order of rotations of k_project_pd_pairs (see k_project_pd_warp)
     if constexpr (std::is_same<T, float>::value) {
+        // 30 x 30 in float keeps the order of rotations of k_project_pd_pairs (see k_project_pd_warp)
         if (N == 30) {
             launch_project_pd_pairs<30, false>(H, count, eps, mirroring, not_converged, sel, s);
             return;
         }
-    }
-    if (N == 12 && scratch.fallback && scratch.n_fallback) {
-        const bool split = scratch.pending && scratch.n_pending;
-        const cudaError_t e = cudaMemsetAsync(scratch.n_fallback, 0, sizeof(unsigned long long), s);
-        if (e != cudaSuccess) throw std::runtime_error(std::string("symx_gb300: memset: ") + cudaGetErrorString(e));
-        if (split) {
-            const cudaError_t e2 = cudaMemsetAsync(scratch.n_pending, 0, sizeof(unsigned long long), s);
-            if (e2 != cudaSuccess) throw std::runtime_error(std::string("symx_gb300: memset: ") + cudaGetErrorString(e2));
-        }
-        if (split) {
+        if (N == 12 && scratch.fallback && scratch.n_fallback && scratch.pending && scratch.n_pending) {
+            for (unsigned long long* c : {scratch.n_fallback, scratch.n_pending}) {
+                const cudaError_t e = cudaMemsetAsync(c, 0, sizeof(unsigned long long), s);
+                if (e != cudaSuccess) throw std::runtime_error(std::string("symx_gb300: memset: ") + cudaGetErrorString(e));
+            }
             k_project_pd_sort<T, 12><<<blocks_for(count, 128), 128, 0, s>>>(H, count, scratch.fallback, scratch.n_fallback,
                                                                            sel, scratch.pending, scratch.n_pending);
             check_launch("project_pd_sort");
-        } else {
-            k_project_pd_deflated<T, 12><<<blocks_for(count, 128), 128, 0, s>>>(H, count, eps, mirroring, not_converged,
-                                                                                  scratch.fallback, scratch.n_fallback, sel);
-            check_launch("project_pd_deflated");
-        }
-        if (split) {
             const unsigned pending_grid = resident_grid(k_project_pd_deflated_listed<T, 12>, 128);
             k_project_pd_deflated_listed<T, 12><<<pending_grid, 128, 0, s>>>(H, scratch.pending, scratch.n_pending, eps,
                                                                            mirroring, not_converged);
             check_launch("project_pd_deflated_listed");
+            const unsigned listed_grid = resident_grid(k_project_pd_listed<T, 12>, 128);
+            k_project_pd_listed<T, 12><<<listed_grid, 128, 0, s>>>(H, scratch.fallback, scratch.n_fallback, eps, mirroring,
+                                                                   not_converged);
+            check_launch("project_pd_listed");
+            return;
         }
-        const unsigned listed_grid = resident_grid(k_project_pd_listed<T, 12>, 128);
-        k_project_pd_listed<T, 12><<<listed_grid, 128, 0, s>>>(H, scratch.fallback, scratch.n_fallback, eps, mirroring,
-                                                               not_converged);
-        check_launch("project_pd_listed");
-        return;
+        if (N == 12) {
+            k_project_pd_unrolled<T, 12><<<blocks_for(count, 128), 128, 0, s>>>(H, count, eps, mirroring, not_converged, sel);
+            check_launch("project_pd");
+            return;
+        }
     }
     switch (N) {
         case 3: k_project_pd_unrolled<T, 3><<<blocks_for(count, 128), 128, 0, s>>>(H, count, eps, mirroring, not_converged, sel); break;
         case 6: k_project_pd_unrolled<T, 6><<<blocks_for(count, 128), 128, 0, s>>>(H, count, eps, mirroring, not_converged, sel); break;
         case 9: k_project_pd_unrolled<T, 9><<<blocks_for(count, 128), 128, 0, s>>>(H, count, eps, mirroring, not_converged, sel); break;
-        case 12: k_project_pd_unrolled<T, 12><<<blocks_for(count, 128), 128, 0, s>>>(H, count, eps, mirroring, not_converged, sel); break;
         default:
             if (N > 30 || N % 3 != 0) throw std::runtime_error("symx_gb300: projection supports N = 3k <= 30");
             k_project_pd_generic<T><<<blocks_for(count, 64), 64, 0, s>>>(H, N, count, eps, mirroring, not_converged, sel);

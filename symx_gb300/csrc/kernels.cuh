@@ -66,14 +66,11 @@ void launch_dot_mixed(const T* a, const double* b, int64_t n, double* partials, 
                       cudaStream_t s);
 
 // Element-Hessian projection, in place, block-major storage, `count` matrices of N x N.
-// not_converged: one int, set to 1 if any matrix hit the sweep cap.  With scratch (12 x 12
-// only: `fallback` holds `count` indices, `n_fallback` one counter), translation-invariant
-// matrices are projected in the 9-dimensional complement of the rigid translations and the
-// others with the full decomposition in a second launch; without it, every matrix takes the
-// full decomposition.
-// 12 x 12 projection lists (each sized for every matrix of one launch): matrices that are not
-// translation-invariant (full decomposition), and, when given, translation-invariant ones
-// whose deflated part is not positive definite (deflated decomposition in full warps).
+// not_converged: one int, set to 1 if any matrix hit the sweep cap.
+// Lists of the 12 x 12 projection in float and of the refined one (each sized for every matrix of one
+// launch): matrices that are not translation-invariant (full decomposition), and
+// translation-invariant ones whose deflated part is not positive definite (deflated decomposition
+// in full warps).  Without them a thread tests and decomposes its matrix in one go.
 struct ProjectionScratch {
     int64_t* fallback = nullptr;
     unsigned long long* n_fallback = nullptr;
