@@ -870,8 +870,8 @@ __device__ __forceinline__ T half_warp_transpose_sum(const T (&a)[3], const T (&
 // thread block streams the blocks of its rows in storage order, kSpmvUnroll per thread with all their
 // loads in flight, leaves the products in shared memory, and sums them with four lanes per row.  (With
 // half a warp per row, 16 lanes for about 15 blocks, too few loads were in flight: 4.0 M blocks in
-// float 45.1 us, now 38.1, or 4.4 TB/s; in double 145 and 124 us.)  The gathers of x, three
-// 4-byte loads per block, are what is left.
+// float 45.1 us, now 38.1, or 4.4 TB/s; in double 145 and 124 us.)  What is left is the
+// chain of a chunk's loads, row pointers, then columns and values, then x.
 constexpr int kSpmvBlock = 128, kSpmvRows = kSpmvBlock / 4, kSpmvUnroll = 4, kSpmvChunk = kSpmvBlock * kSpmvUnroll;
 template <typename T, typename L>
 __global__ void __launch_bounds__(kSpmvBlock, sizeof(T) == 4 ? 8 : 4)
