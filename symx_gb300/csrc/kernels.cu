@@ -867,17 +867,19 @@ __device__ __forceinline__ T half_warp_transpose_sum(const T (&a)[3], const T (&
 }
 
 // y = A x (x and y with 3 values per block row, the C ABI layout).  Bound by the matrix's bytes, so a
-// thread block streams the blocks of its rows in storage order, kSpmvUnroll per thread with all their
-// loads in flight, leaves the products in shared memory, and sums them with four lanes per row.  (With
-// half a warp per row, 16 lanes for about 15 blocks, too few loads were in flight: 4.0 M blocks in
-// float 45.1 us, now 38.1, or 4.4 TB/s; in double 145 and 124 us.)  What is left is the
+// thread block streams the blocks of its rows in storage order, two (in double four) per thread with
+// all their loads in flight, leaves the products in shared memory, and sums them with four lanes per
+// row.  (With half a warp per row, 16 lanes for about 15 blocks, too few loads were in flight: 4.0 M blocks in
+// float 45.1 us, now 35.0, or 4.8 TB/s; in double 145 and 124 us.)  What is left is the
 // chain of a chunk's loads, row pointers, then columns and values, then x.
-constexpr int kSpmvBlock = 128, kSpmvRows = kSpmvBlock / 4, kSpmvUnroll = 4, kSpmvChunk = kSpmvBlock * kSpmvUnroll;
+// In float, four per thread and eight blocks per SM take 38.8 us, two and sixteen spill (48 us).
+constexpr int kSpmvBlock = 128, kSpmvRows = kSpmvBlock / 4;
 template <typename T, typename L>
-__global__ void __launch_bounds__(kSpmvBlock, sizeof(T) == 4 ? 8 : 4)
+__global__ void __launch_bounds__(kSpmvBlock, sizeof(T) == 4 ? 12 : 4)
     k_bcsr_spmv(int n_blocks, const int32_t* __restrict__ row_ptr, const int32_t* __restrict__ cols,
                 const T* __restrict__ vals, L lay, const T* __restrict__ x, T* __restrict__ y)
 {
+    constexpr int kSpmvUnroll = sizeof(T) == 4 ? 2 : 4, kSpmvChunk = kSpmvBlock * kSpmvUnroll;
     __shared__ T prod[3][kSpmvChunk];
     const int tid = threadIdx.x, q = tid & 3;
     const int64_t st = lay.step();
@@ -912,16 +914,18 @@ __global__ void __launch_bounds__(kSpmvBlock, sizeof(T) == 4 ? 8 : 4)
         __syncthreads();
         const int e = (int)(min((int64_t)mine_e, base + kSpmvChunk) - base);
         int k = (int)(max((int64_t)mine_b, base) - base) + q;
-        for (; k + 4 < e; k += 8)  // sums of two: as few roundings in sequence as with a lane per block
+        // added as a half-warp's lanes would add up to 16 blocks: eight apart, four, two, one
+        for (; k < e; k += 16) {
+            const bool h4 = k + 4 < e, h8 = k + 8 < e, h12 = k + 12 < e;
 #pragma unroll
-            for (int i = 0; i < 3; ++i) a[i] += prod[i][k] + prod[i][k + 4];
-        if (k < e)
-#pragma unroll
-            for (int i = 0; i < 3; ++i) a[i] += prod[i][k];
+            for (int i = 0; i < 3; ++i)
+                a[i] += (prod[i][k] + (h8 ? prod[i][k + 8] : T(0))) +
+                        ((h4 ? prod[i][k + 4] : T(0)) + (h12 ? prod[i][k + 12] : T(0)));
+        }
         __syncthreads();
     }
 #pragma unroll
-    for (int o = 1; o < 4; o <<= 1) {
+    for (int o = 2; o > 0; o >>= 1) {
 #pragma unroll
         for (int i = 0; i < 3; ++i) a[i] += __shfl_xor_sync(0xffffffffu, a[i], o);
     }

@@ -1,5 +1,5 @@
 """y = A x through symxg_bcsr_spmv_*: row counts around a thread block's 32 rows, empty rows, rows
-longer than the 512 blocks that a thread block streams at a time, against float64.
+longer than the 256 (in double 512) blocks that a thread block streams at a time, against float64.
 
 Tolerance: a row of n terms is summed in some order, so |error| <= (n + 2) u sum |a| |x|, with u
 the unit roundoff of the type (the float64 reference itself adds a few 2^-53 of the same sum)."""
