@@ -413,17 +413,14 @@ template <>
 struct UnitRoundoff<double> {
     static SYMXG_DEVICE double value() { return 1.1102230246251565e-16; }  // 2^-53
 };
+// True when b - shift I has a Cholesky factorization with every pivot above tau.
 template <typename T, int M>
-SYMXG_DEVICE bool positive_definite_by_cholesky(const T (&b)[M * (M + 1) / 2])
+SYMXG_DEVICE bool cholesky_pivots_above(const T (&b)[M * (M + 1) / 2], T shift, T tau)
 {
-    T dmax = T(0);
-#pragma unroll
-    for (int i = 0; i < M; ++i) dmax = fmax(dmax, b[tri<M>(i, i)]);
-    const T tau = T(16 * M) * UnitRoundoff<T>::value() * dmax;
     T u[M * (M + 1) / 2];  // U = L^T: u(k, i) = L(i, k), k <= i
 #pragma unroll
     for (int j = 0; j < M; ++j) {
-        T d = b[tri<M>(j, j)];
+        T d = b[tri<M>(j, j)] - shift;
 #pragma unroll
         for (int k = 0; k < j; ++k) d -= u[tri<M>(k, j)] * u[tri<M>(k, j)];
         if (!(d > tau)) return false;
@@ -437,6 +434,14 @@ SYMXG_DEVICE bool positive_definite_by_cholesky(const T (&b)[M * (M + 1) / 2])
         }
     }
     return true;
+}
+template <typename T, int M>
+SYMXG_DEVICE bool positive_definite_by_cholesky(const T (&b)[M * (M + 1) / 2])
+{
+    T dmax = T(0);
+#pragma unroll
+    for (int i = 0; i < M; ++i) dmax = fmax(dmax, b[tri<M>(i, i)]);
+    return cholesky_pivots_above<T, M>(b, T(0), T(16 * M) * UnitRoundoff<T>::value() * dmax);
 }
 
 // Upper triangle of the symmetric matrix H (block-major; row-major with Rows) into a, and max |entry| into hmax.  A
@@ -501,6 +506,68 @@ SYMXG_DEVICE void deflate_upper(const T (&a)[3 * NB * (3 * NB + 1) / 2], T (&b)[
             }
             b[tri<M>(p, q)] = s;
         }
+}
+
+// ---- positive definiteness of a double matrix, proved by a Cholesky factorization in float
+//
+// Pivots bound no eigenvalue, and rounding to float moves each by up to 1e-7 of the matrix, so a float
+// factorization of the matrix itself proves nothing about it.  One of F - sigma I does when sigma covers
+// every rounding error (S. M. Rump, "Verification of positive definiteness", BIT Numer. Math. 46 (2006)
+// 433-452).  For an M x M matrix whose float copy F has been factored, with u = 2^-24:
+//   * the factorization: the computed factor satisfies |F' - L L^T| <= gamma_(M + 2) |L| |L^T|, F' =
+//     fl(F - sigma I) (M + 2 and not M + 1: multiplying by a rounded reciprocal root takes two
+//     roundings more than a division), whose norm is at most (M + 2) u trace(F) to first order;
+//   * the diagonal of F': u trace(F);
+//   * F itself: an entrywise relative error k u of the terms of each entry is at most
+//     k u |F|_Frobenius times the norm of the transformation, and |F|_Frobenius <= trace(F) (1 + 2 M u)
+//     once the factorization exists.
+// DefiniteShift is the sum in units of u trace(F), with four units left for the second-order terms and the
+// rounding of the trace.
+template <int M>
+struct DefiniteShift {
+    // F rounded entry by entry from double (k = 1)
+    static constexpr float converted = M + 2 + 1 + 1 + 4;
+    // M = 9: F = Q^T H Q formed in float from the rounded H.  A term has k = 15 roundings (one of the entry,
+    // and per sum three of its coefficient, one of the product, three of the additions); | |Q| |^2 is at
+    // most its column sum 3 / sqrt(3) times its row sum 1 / sqrt(2) + 1 / sqrt(6) + 1 / sqrt(12), below
+    // 2.44: 36.6
+    static constexpr float deflated = M + 2 + 1 + 37 + 4;
+};
+
+// 0: every eigenvalue of H in the complement of the translations is positive, 1: to be decomposed
+// there, 2: not translation-invariant.  H: 12 x 12 in double, block-major (row-major with Rows).
+template <bool Rows>
+SYMXG_DEVICE int classify12(const double* __restrict__ h)
+{
+    constexpr int N = 12, NB = 4, M = 9;
+    float a[N * (N + 1) / 2];
+    double hmax = 0.0, res = 0.0;
+    bool nan = false;
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+        double acc[3] = {0.0, 0.0, 0.0};
+#pragma unroll
+        for (int j = 0; j < N; ++j) {
+            const double v = h[h_index<N, Rows>(i, j)];
+            if (i <= j) a[tri<N>(i, j)] = (float)v;
+            hmax = fmax(hmax, fabs(v));
+            acc[j % 3] += v;
+        }
+#pragma unroll
+        for (int e = 0; e < 3; ++e) {
+            nan |= acc[e] != acc[e];
+            res = fmax(res, fabs(acc[e]));
+        }
+    }
+    if (nan || !(res <= DeflationTol<double>::value() * hmax)) return 2;
+    if (!(hmax > 1e-15 && hmax < 1e15)) return 1;  // float products could leave float's range
+    float b[M * (M + 1) / 2];
+    deflate_upper<float, NB>(a, b);
+    float trace = 0.0f;
+#pragma unroll
+    for (int i = 0; i < M; ++i) trace += b[tri<M>(i, i)];
+    const float shift = DefiniteShift<M>::deflated * UnitRoundoff<float>::value() * trace;
+    return cholesky_pivots_above<float, M>(b, shift, 0.0f) ? 0 : 1;
 }
 
 // b = Q^T H Q (upper triangle) of a translation-invariant H; returns false (b unset) when the

@@ -10,9 +10,10 @@
 //   1. When H annihilates the rigid translations (every elastic energy's does, up to rounding), it
 //      is deflated: B = Q^T H Q, Q the Helmert basis of the node space orthogonal to (1, ..., 1)
 //      (x) I3, M = N - 3.  Otherwise B = H, M = N.
-//   2. A Cholesky factorization of the deflated B in float with pivots above 16 M u of its largest
-//      diagonal entry: H is positive definite in the complement and stays as it is (the
-//      projection would lift the translations' eigenvalues from 0 to eps, below H's rounding).
+//   2. A Cholesky factorization of the deflated B in float.  With pivots above 16 M u of its largest
+//      diagonal entry (float), or of B less a bound of all rounding errors (double: then B is proved
+//      to be positive definite), H stays as it is (the projection would lift the translations'
+//      eigenvalues from 0 to eps).
 //   3. Cyclic Jacobi of B in float (jacobi_sweeps).
 //   4. double: the float eigenvectors X precondition the double decomposition.  X is
 //      orthonormalized in double, X <- X (I - E / 2 + 3/8 E^2) with E = X^T X - I (the series of
@@ -376,8 +377,9 @@ __device__ __forceinline__ bool load_and_deflate(const T* __restrict__ h, const 
     return invariant;
 }
 
-// True when a float copy of the M x M matrix B (row stride LD) has a Cholesky factorization with
-// every pivot above 16 M u of its largest diagonal entry.  f: M x M floats, stride LD.  One warp.
+// Float: true when the M x M matrix B (row stride LD) has a Cholesky factorization with every pivot
+// above 16 M u of its largest diagonal entry.  Double: true when a float one proves that every
+// eigenvalue of B is positive (DefiniteShift).  f: M x M floats, stride LD.  One warp.
 template <typename T, int M, int LD>
 __device__ __forceinline__ bool positive_definite(const T* B, float* f, int lane)
 {
@@ -386,10 +388,19 @@ __device__ __forceinline__ bool positive_definite(const T* B, float* f, int lane
         if (i >= j) f[i * LD + j] = (float)B[i * LD + j];
     }
     __syncwarp();
-    float dmax = lane < M ? f[lane * LD + lane] : 0.f;
+    const float u = symxg_dev::UnitRoundoff<float>::value();
+    float d0 = lane < M ? f[lane * LD + lane] : 0.f, tau = 0.f;
+    if constexpr (sizeof(T) == 4) {
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) dmax = fmaxf(dmax, __shfl_xor_sync(0xffffffffu, dmax, o));
-    const float tau = 16.f * M * symxg_dev::UnitRoundoff<float>::value() * dmax;
+        for (int o = 16; o > 0; o >>= 1) d0 = fmaxf(d0, __shfl_xor_sync(0xffffffffu, d0, o));
+        tau = 16.f * M * u * d0;
+    } else {
+        float trace = d0;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) trace += __shfl_xor_sync(0xffffffffu, trace, o);
+        if (lane < M) f[lane * LD + lane] = d0 - symxg_dev::DefiniteShift<M>::converted * u * trace;
+        __syncwarp();
+    }
     for (int j = 0; j < M; ++j) {
         const float d = f[j * LD + j];  // the same value in every lane
         if (!(d > tau)) return false;
@@ -696,38 +707,6 @@ __global__ void __launch_bounds__(WarpCfg<T, N>::warps * 32, WarpCfg<T, N>::min_
 // the 19,456 that fill the chip once.
 constexpr int kTileThreads = 128;
 
-// 0: positive definite in the complement of the translations, 1: to be decomposed there, 2: not
-// translation-invariant.
-template <bool Rows>
-__device__ __forceinline__ int classify12(const double* __restrict__ h)
-{
-    constexpr int N = 12, NB = 4, M = 9;
-    float a[N * (N + 1) / 2];
-    double hmax = 0.0, res = 0.0;
-    bool nan = false;
-#pragma unroll
-    for (int i = 0; i < N; ++i) {
-        double acc[3] = {0.0, 0.0, 0.0};
-#pragma unroll
-        for (int j = 0; j < N; ++j) {
-            const double v = h[symxg_dev::h_index<N, Rows>(i, j)];
-            if (i <= j) a[symxg_dev::tri<N>(i, j)] = (float)v;
-            hmax = fmax(hmax, fabs(v));
-            acc[j % 3] += v;
-        }
-#pragma unroll
-        for (int e = 0; e < 3; ++e) {
-            nan |= acc[e] != acc[e];
-            res = fmax(res, fabs(acc[e]));
-        }
-    }
-    if (nan || !(res <= symxg_dev::DeflationTol<double>::value() * hmax)) return 2;
-    if (!(hmax > 1e-15 && hmax < 1e15)) return 1;  // float products could leave float's range
-    float b[M * (M + 1) / 2];
-    symxg_dev::deflate_upper<float, NB>(a, b);
-    return symxg_dev::positive_definite_by_cholesky<float, M>(b) ? 0 : 1;
-}
-
 template <bool Rows>
 __global__ void __launch_bounds__(kTileThreads, 3)
     k_project_pd_tile12(double* __restrict__ H, int64_t count, int tile, double eps, int mirroring, int* not_converged,
@@ -745,7 +724,7 @@ __global__ void __launch_bounds__(kTileThreads, 3)
         __syncthreads();
         if (tid < tile && base + tid < count) {
             const int64_t m = sel ? sel[base + tid] : base + tid;
-            const int c = classify12<Rows>(H + m * (N * N));
+            const int c = symxg_dev::classify12<Rows>(H + m * (N * N));
             if (c) list[c - 1][atomicAdd(&n_list[c - 1], 1)] = m;
         }
         __syncthreads();
