@@ -213,7 +213,9 @@ int64_t symxg_wait_poll_limit(void);
 /* Project `count` symmetric n x n matrices (n = 3k <= 30), stored block-major (3x3 block
  * (a,b) at offset (a*k+b)*9, row-major inside), in place.  not_converged: device int set
  * to 1 if a Jacobi sweep cap was hit.  Replaces project_to_PD_inplace
- * (symx/src/solver/second_order/project_to_PD.cpp:12-81).  n = 3..12 run one matrix per
+ * (symx/src/solver/second_order/project_to_PD.cpp:12-81).  A matrix that annihilates the rigid
+ * translations of its n / 3 nodes (n = 12, 18, 24, 30) and has no other eigenvalue below eps is left as it
+ * is: its translations' zero eigenvalues are lifted to eps only along with others.  n = 3..12 run one matrix per
  * thread in registers (n = 12 in f64: ten lanes per matrix), n = 18, 24, 30 one matrix per warp
  * in shared memory.  n = 15, 21, 27
  * run one matrix per thread with the matrix and its eigenvectors in local memory: the first

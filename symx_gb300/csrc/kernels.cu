@@ -164,13 +164,13 @@ __global__ void __launch_bounds__(128) k_project_pd_unrolled(T* __restrict__ H, 
     if (nc) *not_converged = 1;
 }
 
-// Sorting pass of the 12 x 12 projection: matrices whose deflated part is positive definite
+// Sorting pass of the 12 x 12 projection: matrices whose deflated part has no eigenvalue below eps
 // are done (left as they are: the projection would only lift their translation eigenvalues
 // to eps); the others are listed, translation-invariant ones in `pending` for
 // k_project_pd_deflated_listed and the rest in `fallback` for k_project_pd_listed (counts
 // zeroed before the launch), so the eigen-decompositions run in full warps.
 template <typename T, int N>
-__global__ void __launch_bounds__(128) k_project_pd_sort(const T* __restrict__ H, int64_t count,
+__global__ void __launch_bounds__(128) k_project_pd_sort(const T* __restrict__ H, int64_t count, T eps,
                                                          int64_t* __restrict__ fallback, unsigned long long* n_fallback,
                                                          const int64_t* __restrict__ sel, int64_t* __restrict__ pending,
                                                          unsigned long long* n_pending)
@@ -181,7 +181,7 @@ __global__ void __launch_bounds__(128) k_project_pd_sort(const T* __restrict__ H
     const int64_t m = sel ? sel[k] : k;
     T b[M * (M + 1) / 2];
     if (!symxg_dev::deflate_translations<T, N / 3>(H + m * (N * N), b)) fallback[atomicAdd(n_fallback, 1ull)] = m;
-    else if (!symxg_dev::positive_definite_by_cholesky<T, M>(b)) pending[atomicAdd(n_pending, 1ull)] = m;
+    else if (!symxg_dev::eigenvalues_above_by_cholesky<T, M>(b, eps)) pending[atomicAdd(n_pending, 1ull)] = m;
 }
 
 // The deflated eigen-decomposition of the matrices k_project_pd_sort listed as pending
@@ -457,14 +457,14 @@ __device__ __forceinline__ float warp_allmax(float v)
 }
 
 // Warp test of one N x N element Hessian A (shared memory, row stride LD): true when A is
-// translation-invariant (max |A t| <= tol max |A|) and Q^T A Q (Q the Helmert basis of the
+// translation-invariant (max |A t| <= tol max |A|) and Q^T A Q - eps I (Q the Helmert basis of the
 // node space orthogonal to (1, ..., 1), (x) I3) has a Cholesky factorization with pivots above
-// 16 M u of its largest diagonal entry.  A is then positive definite in the complement of the
-// translations up to rounding, and the reference's projection would only lift the three
-// translation eigenvalues from 0 to eps, a change below the rounding of A's entries.  B (the
+// 16 M u of the largest diagonal entry of Q^T A Q.  A's eigenvalues in the complement of the
+// translations are then at least eps up to rounding, and the reference's projection would only lift
+// the three translation eigenvalues from 0 to eps.  B (the
 // same shape) is scratch; every decision is taken by all lanes alike.
 template <int N, int LD>
-__device__ bool pairs_pd_shortcut(const float* __restrict__ A, float* __restrict__ B, int lane)
+__device__ bool pairs_pd_shortcut(const float* __restrict__ A, float* __restrict__ B, float eps, int lane)
 {
     constexpr int NB = N / 3, M = N - 3;
     // rows of A Q (lane i < N: row i): prefix sums over the node blocks; the full sums are
@@ -503,6 +503,8 @@ __device__ bool pairs_pd_shortcut(const float* __restrict__ A, float* __restrict
     // Cholesky (lower triangle, in place): lane i holds row i
     const float dmax = warp_allmax(lane < M ? B[lane * LD + lane] : 0.0f);
     const float tau = float(16 * M) * symxg_dev::UnitRoundoff<float>::value() * dmax;
+    if (lane < M) B[lane * LD + lane] -= fmaxf(eps, 0.0f);
+    __syncwarp();
     for (int j = 0; j < M; ++j) {
         const float d = B[j * LD + j];  // the same value in every lane
         if (!(d > tau)) return false;
@@ -584,7 +586,7 @@ __global__ void __launch_bounds__(ProjPairsCfg<N>::warps * 32, ProjPairsCfg<N>::
         for (int i = w; i < n; i += W) {
             load(at(i));
             // positive definite ones stay as they are
-            if (!pairs_pd_shortcut<N, LD>(A, sB, lane) && lane == 0) list[atomicAdd(&n_list, 1)] = (short)i;
+            if (!pairs_pd_shortcut<N, LD>(A, sB, eps, lane) && lane == 0) list[atomicAdd(&n_list, 1)] = (short)i;
             __syncwarp();
         }
         __syncthreads();
@@ -2870,7 +2872,7 @@ void launch_project_pd(T* H, int N, int64_t count, T eps, bool mirroring, int* n
                 const cudaError_t e = cudaMemsetAsync(c, 0, sizeof(unsigned long long), s);
                 if (e != cudaSuccess) throw std::runtime_error(std::string("symx_gb300: memset: ") + cudaGetErrorString(e));
             }
-            k_project_pd_sort<T, 12><<<blocks_for(count, 128), 128, 0, s>>>(H, count, scratch.fallback, scratch.n_fallback,
+            k_project_pd_sort<T, 12><<<blocks_for(count, 128), 128, 0, s>>>(H, count, (T)eps, scratch.fallback, scratch.n_fallback,
                                                                            sel, scratch.pending, scratch.n_pending);
             check_launch("project_pd_sort");
             const unsigned pending_grid = resident_grid(k_project_pd_deflated_listed<T, 12>, 128);
@@ -2932,7 +2934,7 @@ void launch_project_pd_refined12(T* H, int64_t count, double eps, bool mirroring
         const cudaError_t e = cudaMemsetAsync(c, 0, sizeof(unsigned long long), s);
         if (e != cudaSuccess) throw std::runtime_error(std::string("symx_gb300: memset: ") + cudaGetErrorString(e));
     }
-    k_project_pd_sort<T, 12><<<blocks_for(count, 128), 128, 0, s>>>(H, count, scratch.fallback, scratch.n_fallback, sel,
+    k_project_pd_sort<T, 12><<<blocks_for(count, 128), 128, 0, s>>>(H, count, (T)eps, scratch.fallback, scratch.n_fallback, sel,
                                                                    scratch.pending, scratch.n_pending);
     check_launch("project_pd_sort");
     const unsigned pending_grid = resident_grid(k_project_pd_refined_listed<T, 12, true>, 64);

@@ -400,9 +400,9 @@ SYMXG_DEVICE T helmert(const T (&c)[NB], int i, int m)
     return i < m ? c[m] : (i == m ? -T(m) * c[m] : T(0));
 }
 
-// True when the symmetric M x M matrix b (upper triangle) has a Cholesky factorization whose
-// pivots all exceed 16 M u of its largest diagonal entry (u the unit roundoff of T): it is
-// then positive definite up to rounding, with every eigenvalue above -(rounding of b).
+// True when b - max(eps, 0) I, b a symmetric M x M matrix (upper triangle), has a Cholesky factorization
+// whose pivots all exceed 16 M u of b's largest diagonal entry (u the unit roundoff of T): every
+// eigenvalue of b is then at least max(eps, 0) up to the rounding of b.
 template <typename T>
 struct UnitRoundoff;
 template <>
@@ -436,12 +436,12 @@ SYMXG_DEVICE bool cholesky_pivots_above(const T (&b)[M * (M + 1) / 2], T shift, 
     return true;
 }
 template <typename T, int M>
-SYMXG_DEVICE bool positive_definite_by_cholesky(const T (&b)[M * (M + 1) / 2])
+SYMXG_DEVICE bool eigenvalues_above_by_cholesky(const T (&b)[M * (M + 1) / 2], T eps)
 {
     T dmax = T(0);
 #pragma unroll
     for (int i = 0; i < M; ++i) dmax = fmax(dmax, b[tri<M>(i, i)]);
-    return cholesky_pivots_above<T, M>(b, T(0), T(16 * M) * UnitRoundoff<T>::value() * dmax);
+    return cholesky_pivots_above<T, M>(b, fmax(eps, T(0)), T(16 * M) * UnitRoundoff<T>::value() * dmax);
 }
 
 // Upper triangle of the symmetric matrix H (block-major; row-major with Rows) into a, and max |entry| into hmax.  A
@@ -508,16 +508,16 @@ SYMXG_DEVICE void deflate_upper(const T (&a)[3 * NB * (3 * NB + 1) / 2], T (&b)[
         }
 }
 
-// ---- positive definiteness of a double matrix, proved by a Cholesky factorization in float
+// ---- eigenvalues of a double matrix above eps, proved by a Cholesky factorization in float
 //
 // Pivots bound no eigenvalue, and rounding to float moves each by up to 1e-7 of the matrix, so a float
-// factorization of the matrix itself proves nothing about it.  One of F - sigma I does when sigma covers
-// every rounding error (S. M. Rump, "Verification of positive definiteness", BIT Numer. Math. 46 (2006)
+// factorization of the matrix itself proves nothing about it.  One of F - (eps + sigma) I does when sigma
+// covers every rounding error (S. M. Rump, "Verification of positive definiteness", BIT Numer. Math. 46 (2006)
 // 433-452).  For an M x M matrix whose float copy F has been factored, with u = 2^-24:
 //   * the factorization: the computed factor satisfies |F' - L L^T| <= gamma_(M + 2) |L| |L^T|, F' =
-//     fl(F - sigma I) (M + 2 and not M + 1: multiplying by a rounded reciprocal root takes two
+//     fl(F - (eps + sigma) I) (M + 2 and not M + 1: multiplying by a rounded reciprocal root takes two
 //     roundings more than a division), whose norm is at most (M + 2) u trace(F) to first order;
-//   * the diagonal of F': u trace(F);
+//   * the diagonal of F' and the sum eps + sigma: 3 u trace(F), eps being below the diagonal;
 //   * F itself: an entrywise relative error k u of the terms of each entry is at most
 //     k u |F|_Frobenius times the norm of the transformation, and |F|_Frobenius <= trace(F) (1 + 2 M u)
 //     once the factorization exists.
@@ -526,18 +526,18 @@ SYMXG_DEVICE void deflate_upper(const T (&a)[3 * NB * (3 * NB + 1) / 2], T (&b)[
 template <int M>
 struct DefiniteShift {
     // F rounded entry by entry from double (k = 1)
-    static constexpr float converted = M + 2 + 1 + 1 + 4;
+    static constexpr float converted = M + 2 + 3 + 1 + 4;
     // M = 9: F = Q^T H Q formed in float from the rounded H.  A term has k = 15 roundings (one of the entry,
     // and per sum three of its coefficient, one of the product, three of the additions); | |Q| |^2 is at
     // most its column sum 3 / sqrt(3) times its row sum 1 / sqrt(2) + 1 / sqrt(6) + 1 / sqrt(12), below
     // 2.44: 36.6
-    static constexpr float deflated = M + 2 + 1 + 37 + 4;
+    static constexpr float deflated = M + 2 + 3 + 37 + 4;
 };
 
-// 0: every eigenvalue of H in the complement of the translations is positive, 1: to be decomposed
+// 0: every eigenvalue of H in the complement of the translations is at least eps, 1: to be decomposed
 // there, 2: not translation-invariant.  H: 12 x 12 in double, block-major (row-major with Rows).
 template <bool Rows>
-SYMXG_DEVICE int classify12(const double* __restrict__ h)
+SYMXG_DEVICE int classify12(const double* __restrict__ h, double eps)
 {
     constexpr int N = 12, NB = 4, M = 9;
     float a[N * (N + 1) / 2];
@@ -566,7 +566,7 @@ SYMXG_DEVICE int classify12(const double* __restrict__ h)
     float trace = 0.0f;
 #pragma unroll
     for (int i = 0; i < M; ++i) trace += b[tri<M>(i, i)];
-    const float shift = DefiniteShift<M>::deflated * UnitRoundoff<float>::value() * trace;
+    const float shift = DefiniteShift<M>::deflated * UnitRoundoff<float>::value() * trace + (float)fmax(eps, 0.0);
     return cholesky_pivots_above<float, M>(b, shift, 0.0f) ? 0 : 1;
 }
 
@@ -665,17 +665,16 @@ SYMXG_DEVICE int project_deflated_finish(T* __restrict__ H, T (&b)[(3 * NB - 3) 
     return 1;
 }
 
-// Q^T H Q positive definite (the usual case for an elastic element near its rest shape): the
-// projection keeps its eigenvalues and only lifts the three translation eigenvalues from 0 to
-// eps (the term eps / NB (1 1^T (x) I3)), a change far below the rounding of H's entries, so
-// H is left as it is and the eigen-decomposition is skipped.
+// Every eigenvalue of Q^T H Q at least eps (the usual case for an elastic element near its rest
+// shape): the projection keeps them and would only lift the three translation eigenvalues from 0 to
+// eps (the term eps / NB (1 1^T (x) I3)); H is left as it is and the eigen-decomposition is skipped.
 template <typename T, int NB>
 SYMXG_DEVICE int project_pd_deflated(T* __restrict__ H, T eps, bool mirroring, int* not_converged)
 {
     constexpr int M = 3 * NB - 3;
     T b[M * (M + 1) / 2];
     if (!deflate_translations<T, NB>(H, b)) return -1;
-    if (positive_definite_by_cholesky<T, M>(b)) return 0;
+    if (eigenvalues_above_by_cholesky<T, M>(b, eps)) return 0;
     return project_deflated_finish<T, NB>(H, b, eps, mirroring, not_converged);
 }
 

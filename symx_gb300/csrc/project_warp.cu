@@ -10,10 +10,10 @@
 //   1. When H annihilates the rigid translations (every elastic energy's does, up to rounding), it
 //      is deflated: B = Q^T H Q, Q the Helmert basis of the node space orthogonal to (1, ..., 1)
 //      (x) I3, M = N - 3.  Otherwise B = H, M = N.
-//   2. A Cholesky factorization of the deflated B in float.  With pivots above 16 M u of its largest
-//      diagonal entry (float), or of B less a bound of all rounding errors (double: then B is proved
-//      to be positive definite), H stays as it is (the projection would lift the translations'
-//      eigenvalues from 0 to eps).
+//   2. A Cholesky factorization of B - eps I in float (B deflated).  With pivots above 16 M u of B's
+//      largest diagonal entry (float), or when it stands a further shift by a bound of all rounding
+//      errors (double: no eigenvalue of B is below eps then), H stays as it is (the projection would
+//      only lift the translations' eigenvalues from 0 to eps).
 //   3. Cyclic Jacobi of B in float (jacobi_sweeps).
 //   4. double: the float eigenvectors X precondition the double decomposition.  X is
 //      orthonormalized in double, X <- X (I - E / 2 + 3/8 E^2) with E = X^T X - I (the series of
@@ -377,11 +377,11 @@ __device__ __forceinline__ bool load_and_deflate(const T* __restrict__ h, const 
     return invariant;
 }
 
-// Float: true when the M x M matrix B (row stride LD) has a Cholesky factorization with every pivot
-// above 16 M u of its largest diagonal entry.  Double: true when a float one proves that every
-// eigenvalue of B is positive (DefiniteShift).  f: M x M floats, stride LD.  One warp.
+// Float: true when B - eps I (M x M, row stride LD) has a Cholesky factorization with every pivot
+// above 16 M u of B's largest diagonal entry.  Double: true when a float one proves that every
+// eigenvalue of B is at least eps (DefiniteShift).  f: M x M floats, stride LD.  One warp.
 template <typename T, int M, int LD>
-__device__ __forceinline__ bool positive_definite(const T* B, float* f, int lane)
+__device__ __forceinline__ bool eigenvalues_above(const T* B, float* f, float eps, int lane)
 {
     for (int idx = lane; idx < M * M; idx += 32) {
         const int i = idx / M, j = idx % M;
@@ -389,18 +389,21 @@ __device__ __forceinline__ bool positive_definite(const T* B, float* f, int lane
     }
     __syncwarp();
     const float u = symxg_dev::UnitRoundoff<float>::value();
-    float d0 = lane < M ? f[lane * LD + lane] : 0.f, tau = 0.f;
+    const float d0 = lane < M ? f[lane * LD + lane] : 0.f;
+    float shift = fmaxf(eps, 0.f), tau = 0.f;
     if constexpr (sizeof(T) == 4) {
+        float dmax = d0;
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) d0 = fmaxf(d0, __shfl_xor_sync(0xffffffffu, d0, o));
-        tau = 16.f * M * u * d0;
+        for (int o = 16; o > 0; o >>= 1) dmax = fmaxf(dmax, __shfl_xor_sync(0xffffffffu, dmax, o));
+        tau = 16.f * M * u * dmax;
     } else {
         float trace = d0;
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) trace += __shfl_xor_sync(0xffffffffu, trace, o);
-        if (lane < M) f[lane * LD + lane] = d0 - symxg_dev::DefiniteShift<M>::converted * u * trace;
-        __syncwarp();
+        shift += symxg_dev::DefiniteShift<M>::converted * u * trace;
     }
+    if (lane < M) f[lane * LD + lane] = d0 - shift;
+    __syncwarp();
     for (int j = 0; j < M; ++j) {
         const float d = f[j * LD + j];  // the same value in every lane
         if (!(d > tau)) return false;
@@ -679,7 +682,8 @@ __global__ void __launch_bounds__(WarpCfg<T, N>::warps * 32, WarpCfg<T, N>::min_
             const bool invariant = load_and_deflate<T, N, 32, Rows>(at(i), g, lane, true, true, amax, scale);
             bool done = false;
             if (invariant)
-                done = positive_definite<T, N - 3, kStride<N>>(g.b, reinterpret_cast<float*>(sizeof(T) == 8 ? g.s : g.a), lane);
+                done = eigenvalues_above<T, N - 3, kStride<N>>(g.b, reinterpret_cast<float*>(sizeof(T) == 8 ? g.s : g.a),
+                                                               (float)(eps * scale), lane);
             if (!done && lane == 0) list[atomicAdd(&n_list, 1)] = (short)(invariant ? i : -1 - i);
             __syncwarp();
         }
@@ -724,7 +728,7 @@ __global__ void __launch_bounds__(kTileThreads, 3)
         __syncthreads();
         if (tid < tile && base + tid < count) {
             const int64_t m = sel ? sel[base + tid] : base + tid;
-            const int c = symxg_dev::classify12<Rows>(H + m * (N * N));
+            const int c = symxg_dev::classify12<Rows>(H + m * (N * N), eps);
             if (c) list[c - 1][atomicAdd(&n_list[c - 1], 1)] = m;
         }
         __syncthreads();
@@ -782,7 +786,7 @@ __global__ void __launch_bounds__(kTileThreads, 3)
             float b[M * (M + 1) / 2];
             if (!symxg_dev::deflate_translations<float, N / 3, true>(H + m * (N * N), b))
                 work[2 + atomicAdd(work + 1, 1)] = (int)m;
-            else if (!symxg_dev::positive_definite_by_cholesky<float, M>(b))  // those stay as they are
+            else if (!symxg_dev::eigenvalues_above_by_cholesky<float, M>(b, eps))  // those stay as they are
                 list[atomicAdd(&n_list, 1)] = (short)i;
         }
         __syncthreads();

@@ -29,8 +29,8 @@ int main(int argc, char** argv)
         double bm[144];
         for (int i = 0; i < 12; ++i)
             for (int j = 0; j < 12; ++j) bm[symxg_dev::bm_index<12>(i, j)] = h[12 * i + j];
-        out[e] = symxg_dev::classify12<true>(h);
-        out[count + e] = symxg_dev::classify12<false>(bm);
+        out[e] = symxg_dev::classify12<true>(h, 0.0);
+        out[count + e] = symxg_dev::classify12<false>(bm, 0.0);
     }
     std::ofstream g(argv[2], std::ios::binary);
     g.write(reinterpret_cast<const char*>(out.data()), out.size() * sizeof(int32_t));
