@@ -316,10 +316,11 @@ struct GroupMem {
 
 // The matrix h times `scale` into g.a (row-major), amax = max |entry| of it, and g.b = Q^T (scale h) Q
 // (M x M).  Returns whether it is translation-invariant: max |H t| <= tol max |H|.  In double, scale
-// is the power of two that brings amax into [1, 2), so the float stages cannot overflow.
+// is the power of two that brings amax into [1, 2), so the float stages cannot overflow, or a smaller
+// one when eps times it could leave double's range (a matrix that is zero beside eps).
 template <typename T, int N, int L, bool Rows>
 __device__ __forceinline__ bool load_and_deflate(const T* __restrict__ h, const GroupMem<T, N>& g, int gl, bool member,
-                                                 bool work, float& amax, T& scale)
+                                                 bool work, T eps, float& amax, T& scale)
 {
     constexpr int LD = kStride<N>, NB = N / 3, M = N - 3;
     const Helmert<T, NB> hm;
@@ -334,6 +335,7 @@ __device__ __forceinline__ bool load_and_deflate(const T* __restrict__ h, const 
     scale = T(1);
     if constexpr (sizeof(T) == 8) {
         int ex = -1000;
+        if (eps > 0.0 && eps < (double)INFINITY) ex = max(ex, ilogb(eps) - 1000);
         if (hmax > 0.0 && hmax < (double)INFINITY) ex = max(ex, ilogb(hmax));
         ex = (int)group_max<L>((float)(ex + 2000), g.red, gl, member) - 2000;
         scale = scalbn(1.0, -ex);
@@ -679,7 +681,7 @@ __global__ void __launch_bounds__(WarpCfg<T, N>::warps * 32, WarpCfg<T, N>::min_
         if (threadIdx.x == 0) n_list = 0;
         __syncthreads();
         for (int i = w; i < n; i += W) {
-            const bool invariant = load_and_deflate<T, N, 32, Rows>(at(i), g, lane, true, true, amax, scale);
+            const bool invariant = load_and_deflate<T, N, 32, Rows>(at(i), g, lane, true, true, eps, amax, scale);
             bool done = false;
             if (invariant)
                 done = eigenvalues_above<T, N - 3, kStride<N>>(g.b, reinterpret_cast<float*>(sizeof(T) == 8 ? g.s : g.a),
@@ -692,7 +694,7 @@ __global__ void __launch_bounds__(WarpCfg<T, N>::warps * 32, WarpCfg<T, N>::min_
         for (int k = w; k < pending; k += W) {
             const int i = list[k];
             T* h = at(i < 0 ? -1 - i : i);
-            load_and_deflate<T, N, 32, Rows>(h, g, lane, true, true, amax, scale);
+            load_and_deflate<T, N, 32, Rows>(h, g, lane, true, true, eps, amax, scale);
             if (i >= 0)
                 ok = decompose_and_correct<T, N, 32, true, Rows>(h, g, lane, true, true, amax, scale, eps, mirroring != 0) && ok;
             else
@@ -741,7 +743,7 @@ __global__ void __launch_bounds__(kTileThreads, 3)
             double* h = H + (work ? list[0][i0 + grp] : 0) * (N * N);
             float amax;
             double scale;
-            load_and_deflate<double, N, 10, Rows>(h, g, gl, member, work, amax, scale);
+            load_and_deflate<double, N, 10, Rows>(h, g, gl, member, work, eps, amax, scale);
             ok = decompose_and_correct<double, N, 10, true, Rows>(h, g, gl, member, work, amax, scale, eps, mirroring != 0) && ok;
         }
         for (int i0 = turn * 2; i0 < n2; i0 += 2 * W) {
@@ -751,7 +753,7 @@ __global__ void __launch_bounds__(kTileThreads, 3)
             double* h = H + (work ? list[1][i0 + grp] : 0) * (N * N);
             float amax;
             double scale;
-            load_and_deflate<double, N, 16, Rows>(h, g, gl, true, work, amax, scale);
+            load_and_deflate<double, N, 16, Rows>(h, g, gl, true, work, eps, amax, scale);
             ok = decompose_and_correct<double, N, 16, false, Rows>(h, g, gl, true, work, amax, scale, eps, mirroring != 0) && ok;
         }
         __syncthreads();
