@@ -339,6 +339,7 @@ __device__ __forceinline__ bool load_and_deflate(const T* __restrict__ h, const 
         if (hmax > 0.0 && hmax < (double)INFINITY) ex = max(ex, ilogb(hmax));
         ex = (int)group_max<L>((float)(ex + 2000), g.red, gl, member) - 2000;
         scale = scalbn(1.0, -ex);
+        __syncwarp();  // the loop below reads what other lanes stored (group_max<32> orders no memory)
         if (work && scale != 1.0)
             for (int idx = gl; idx < N * N; idx += L) g.a[(idx / N) * LD + idx % N] *= scale;
     }
