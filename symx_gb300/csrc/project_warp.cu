@@ -591,11 +591,20 @@ __device__ __forceinline__ bool decompose_and_correct(T* __restrict__ h, const G
             for (int j = 0; j < M; ++j) w[j] = fma(t, V[j * LD + k], w[j]);
         }
     const T unscale = T(1) / scale;  // a power of two
+    // 12 x 12: both triangles from one value, as in the forms with a thread per matrix
+    constexpr bool both = N == 12;
+    auto add = [&](int i, int j, T correction) {
+        T* const p = h + symxg_dev::h_index<N, Rows>(i, j);
+        const T sum = *p + correction;
+        *p = sum;
+        if (both && i != j) h[symxg_dev::h_index<N, Rows>(j, i)] = sum;
+    };
     __syncwarp();
     if constexpr (!Deflate) {
         if (work && changed && gl < M)
 #pragma unroll
-            for (int j = 0; j < M; ++j) h[Rows ? gl * N + j : ((gl / 3) * NB + j / 3) * 9 + (gl % 3) * 3 + j % 3] += w[j] * unscale;
+            for (int j = 0; j < M; ++j)
+                if (!both || j >= gl) add(gl, j, w[j] * unscale);
     } else {
         // Q w Q^T by suffix sums over the nodes: columns of the own row, then rows of the own columns;
         // the translations' eigenvalues 0 -> eps (0 when mirroring)
@@ -626,14 +635,13 @@ __device__ __forceinline__ bool decompose_and_correct(T* __restrict__ h, const G
                 for (int d = 0; d < 3; ++d) {
                     const T lift = c % 3 == d ? lam_t / T(NB) : T(0);
                     T tail = T(0);
-                    T* const hc = h + (Rows ? d * N + c : (c / 3) * 9 + d * 3 + c % 3);
 #pragma unroll
                     for (int m = NB - 1; m >= 1; --m) {
                         const T t = hm.c[m] * W[(3 * (m - 1) + d) * LD + c];
-                        hc[m * 3 * N] += (tail - T(m) * t + lift) * unscale;
+                        if (!both || 3 * m + d <= c) add(3 * m + d, c, (tail - T(m) * t + lift) * unscale);
                         tail += t;
                     }
-                    hc[0] += (tail + lift) * unscale;
+                    if (!both || d <= c) add(d, c, (tail + lift) * unscale);
                 }
             }
     }
