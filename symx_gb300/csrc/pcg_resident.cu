@@ -123,8 +123,11 @@ constexpr int kSetWords = kSums * (kLevel0Words + kLevel1Words);
 constexpr size_t kSumBytes = sizeof(Word) * 2 * kSetWords;
 static_assert(kSumBytes <= 2 * sizeof(double) * kResidentPartials, "the exchange words fit in the partials");
 
+// Waits are bounded: the first one of a block to run out of polls sets *abort (in shared memory), and
+// every other wait of the block then gives up at its next poll.
 template <typename S>
-__device__ __forceinline__ bool poll_sums(const Word* w, bool mine, unsigned long long tag, S& v, long long max_polls)
+__device__ __forceinline__ bool poll_sums(const Word* w, bool mine, unsigned long long tag, S& v, long long max_polls,
+                                          volatile int* abort)
 {
     for (long long polls = 0; polls < max_polls; ++polls) {
         if (mine) {
@@ -135,7 +138,9 @@ __device__ __forceinline__ bool poll_sums(const Word* w, bool mine, unsigned lon
             }
         }
         if (!__any_sync(0xffffffffu, mine)) return true;
+        if (__any_sync(0xffffffffu, *abort)) return false;  // a vote: the warp leaves together
     }
+    *abort = 1;
     return false;
 }
 template <typename S>
@@ -163,25 +168,22 @@ __device__ __forceinline__ void sum_place(SumPlace& s)
     for (int k = 0; k < s.groups; ++k) s.copy[k] = (m % min(C, G - k * C)) * kGroupStride + k;
 }
 
-// One warp: the grid's total of this block's sum v (lane 0's), valid in lane 0.  False when a
-// wait gave up.
+// One warp: the grid's total of this block's sum v (lane 0's), valid in lane 0 unless a wait gave up.
 template <typename S>
-__device__ __forceinline__ bool grid_sum(const SumPlace& at, Word* level0, Word* level1, unsigned long long tag, S& v,
-                                         long long max_polls)
+__device__ __forceinline__ void grid_sum(const SumPlace& at, Word* level0, Word* level1, unsigned long long tag, S& v,
+                                         long long max_polls, volatile int* abort)
 {
     const int lane = threadIdx.x & 31;
     S t;
     sum_from_bits(0, t);
     if (lane == 0) st_word(level0 + at.own0, sum_bits(v), tag);
-    if (!poll_sums(level0 + at.first0 + lane, lane < at.members, tag, t, max_polls)) return false;
+    if (!poll_sums(level0 + at.first0 + lane, lane < at.members, tag, t, max_polls, abort)) return;
     v = sum16(t);
-    if (at.groups == 1) return true;
+    if (at.groups == 1) return;
     if (lane == 0) st_word(level1 + at.own1, sum_bits(v), tag);
     sum_from_bits(0, t);
     const bool reads = lane < at.groups;
-    if (!poll_sums(level1 + (reads ? at.copy[lane] : 0), reads, tag, t, max_polls)) return false;
-    v = sum16(t);
-    return true;
+    if (poll_sums(level1 + (reads ? at.copy[lane] : 0), reads, tag, t, max_polls, abort)) v = sum16(t);
 }
 
 // Warp sums of eight values, transposing as it goes (a lane keeps half of its values and sends
@@ -335,15 +337,17 @@ __global__ void __launch_bounds__(resident_threads<T>(), 1) k_pcg_resident(PcgBu
     __shared__ S red[kSums][32], total[kSums];
     __shared__ int cut[2], scan[33];
     __shared__ SumPlace place;
+    __shared__ int abort_flag;  // a wait of this block ran out of polls; set at any time
     // scalars of the iteration, thread 0's but for `converged` (in shared memory: the other
-    // threads hold no registers for them)
+    // threads hold no registers for them).  They change only between the barrier of the exchange's
+    // warps and the block's next barrier, so every thread leaves the loop in the same iteration.
     __shared__ struct {
         S rz, pAp;
         double thr_abs, thr_rel;
         T alpha, beta;
         int stop;       // 1: p.Ap <= 0
         int converged;  // 1: converged, 2: out of iterations
-        int gave_up;    // a wait ran out of polls
+        int gave_up;    // abort_flag, as thread 0 found it after the exchange
     } ctl;
     const int tid = threadIdx.x, threads = blockDim.x, lane = tid & 31, warp = tid >> 5;
     const int G = gridDim.x, n = B.n_blocks;
@@ -470,12 +474,13 @@ __global__ void __launch_bounds__(resident_threads<T>(), 1) k_pcg_resident(PcgBu
         ctl.thr_abs = st0.abs_tol * st0.abs_tol * st0.bb;
         ctl.thr_rel = st0.rel_tol * st0.error0 * st0.rel_tol * st0.error0 * st0.bb;
         ctl.alpha = ctl.beta = T(0);
-        ctl.stop = ctl.converged = ctl.gave_up = 0;
+        ctl.stop = ctl.converged = ctl.gave_up = abort_flag = 0;
     }
     __syncthreads();
 
     const int sum_warps = min((3 * R + 31) / 32, threads / 32);
     const long long max_polls = B.staged.max_polls;
+    volatile int* const abort = &abort_flag;
     int it = 0;
     for (;; ++it) {
         const unsigned tag = (unsigned)it + 1u;
@@ -483,8 +488,8 @@ __global__ void __launch_bounds__(resident_threads<T>(), 1) k_pcg_resident(PcgBu
         auto wait_row = [&](int c) {
             Row4<T> z;
             for (long long polls = 0; !read_row(zt, c, tag, z); ++polls)
-                if (polls >= max_polls) {
-                    ctl.gave_up = 1;
+                if (polls >= max_polls || *abort) {
+                    *abort = 1;
                     break;
                 }
             return z;
@@ -554,14 +559,12 @@ __global__ void __launch_bounds__(resident_threads<T>(), 1) k_pcg_resident(PcgBu
                 if (sum_warps > 1) v = sum_add(v, sum_xor(v, 1));
                 Word* level0 = reinterpret_cast<Word*>(B.partials) + (it & 1) * kSetWords;
                 Word* level1 = level0 + kSums * kLevel0Words;
-                const bool ok = grid_sum(place, level0 + warp * kLevel0Words, level1 + warp * kLevel1Words, tag, v, max_polls);
-                if (lane == 0) {
-                    total[warp] = v;
-                    if (!ok) ctl.gave_up = 1;
-                }
+                grid_sum(place, level0 + warp * kLevel0Words, level1 + warp * kLevel1Words, tag, v, max_polls, abort);
+                if (lane == 0) total[warp] = v;
             }
             asm volatile("bar.sync 1, %0;" ::"n"(32 * kSumWarps) : "memory");
             if (tid == 0) {
+                ctl.gave_up = *abort;
                 const T beta = it > 0 ? quotient(total[1], ctl.rz) : T(0);
                 const S pAp = p_dot_q(total[2], total[3], total[4], beta);
                 ctl.beta = beta;
