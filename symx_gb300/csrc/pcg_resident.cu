@@ -470,9 +470,11 @@ __global__ void __launch_bounds__(resident_threads<T>(), 1) k_pcg_resident(PcgBu
     if (tid == 0) {
         sum_from_bits(0, ctl.rz);
         sum_from_bits(0, ctl.pAp);
-        // sqrt(rr / bb) < abs_tol  and  sqrt(rr / bb) / error0 < rel_tol, as comparisons of rr
-        ctl.thr_abs = st0.abs_tol * st0.abs_tol * st0.bb;
-        ctl.thr_rel = st0.rel_tol * st0.error0 * st0.rel_tol * st0.error0 * st0.bb;
+        // sqrt(rr / bb) < abs_tol  and  sqrt(rr / bb) / error0 < rel_tol, as comparisons of rr; rr = 0
+        // passes any positive tolerance, also one whose square is below double's range
+        const double least = 4.9406564584124654e-324;
+        ctl.thr_abs = fmax(st0.abs_tol * st0.abs_tol * st0.bb, st0.abs_tol > 0.0 ? least : 0.0);
+        ctl.thr_rel = fmax(st0.rel_tol * st0.error0 * st0.rel_tol * st0.error0 * st0.bb, st0.rel_tol > 0.0 ? least : 0.0);
         ctl.alpha = ctl.beta = T(0);
         ctl.stop = ctl.converged = ctl.gave_up = abort_flag = 0;
     }
