@@ -337,6 +337,7 @@ __global__ void __launch_bounds__(resident_threads<T>(), 1) k_pcg_resident(PcgBu
     __shared__ S red[kSums][32], total[kSums];
     __shared__ int cut[2], scan[33];
     __shared__ SumPlace place;
+    __shared__ int b_exponent;
     __shared__ int abort_flag;  // a wait of this block ran out of polls; set at any time
     // scalars of the iteration, thread 0's but for `converged` (in shared memory: the other
     // threads hold no registers for them).  They change only between the barrier of the exchange's
@@ -351,7 +352,14 @@ __global__ void __launch_bounds__(resident_threads<T>(), 1) k_pcg_resident(PcgBu
     } ctl;
     const int tid = threadIdx.x, threads = blockDim.x, lane = tid & 31, warp = tid >> 5;
     const int G = gridDim.x, n = B.n_blocks;
-    if (tid == 0) st0 = *B.state;
+    if (tid == 0) {
+        st0 = *B.state;
+        // The solve runs on b / 2^k with |b| about 2^k, exactly: the sums over all rows, in float's range
+        // for float, then neither overflow nor vanish for any b that its type holds.
+        constexpr int limit = sizeof(T) == 4 ? 120 : 1000;
+        b_exponent = st0.bb > 0.0 && st0.bb < (double)INFINITY ? min(max(ilogb(st0.bb) / 2, -limit), limit) : 0;
+        st0.bb = scalbn(st0.bb, -2 * b_exponent);
+    }
     if (tid == 64) sum_place(place);
     if (warp < 2) {
         const int r = block_first_row(blockIdx.x + warp, G, n, B.row_ptr);
@@ -374,9 +382,12 @@ __global__ void __launch_bounds__(resident_threads<T>(), 1) k_pcg_resident(PcgBu
     for (int i = tid; i <= rows; i += threads) rp[i] = B.row_ptr[row0 + i];
     for (int j = tid; j < 3 * R; j += threads) sx[j] = sr[j] = sz[j] = sp[j] = sq[j] = sw[j] = T(0);
     __syncthreads();
+    const T to_unit = (T)scalbn(1.0, -b_exponent), from_unit = (T)scalbn(1.0, b_exponent);
     for (int i = tid; i < rows; i += threads) {
         const int64_t g = row0 + i;
-        const Row4<T> r = ld4(B.r + 4 * g), z = ld4(B.z + 4 * g);
+        Row4<T> r = ld4(B.r + 4 * g), z = ld4(B.z + 4 * g);
+        r = Row4<T>{r.x * to_unit, r.y * to_unit, r.z * to_unit, T(0)};
+        z = Row4<T>{z.x * to_unit, z.y * to_unit, z.z * to_unit, T(0)};
         publish_row(zt, row0 + i, z, 1u);
         sr[i] = r.x;
         sr[R + i] = r.y;
@@ -630,7 +641,7 @@ __global__ void __launch_bounds__(resident_threads<T>(), 1) k_pcg_resident(PcgBu
         if (!halo) __syncthreads();  // the next product writes w
     }
     for (int i = tid; i < rows; i += threads)
-        st4(B.x + 4 * (int64_t)(row0 + i), Row4<T>{sx[i], sx[R + i], sx[2 * R + i], T(0)});
+        st4(B.x + 4 * (int64_t)(row0 + i), Row4<T>{sx[i] * from_unit, sx[R + i] * from_unit, sx[2 * R + i] * from_unit, T(0)});
     if (ctl.gave_up) {
         if (tid == 0) atomicExch(&B.state->wait_failed, 1);
         return;
@@ -642,11 +653,11 @@ __global__ void __launch_bounds__(resident_threads<T>(), 1) k_pcg_resident(PcgBu
         st->converged = ctl.converged == 1;
         st->indefinite = indefinite;
         st->done = 1;
-        st->pAp = sum_value(ctl.pAp);
+        st->pAp = scalbn(sum_value(ctl.pAp), 2 * b_exponent);
         st->alpha = ctl.alpha;
         st->beta = ctl.beta;
-        st->rz = sum_value(ctl.rz);
-        st->rr = sum_value(total[0]);
+        st->rz = scalbn(sum_value(ctl.rz), 2 * b_exponent);
+        st->rr = scalbn(sum_value(total[0]), 2 * b_exponent);
         st->error = it > 0 ? sqrt(sum_value(total[0]) / st0.bb) : st0.error;
     }
 }
