@@ -23,12 +23,14 @@ void ck(cudaError_t e, const char* what)
 // Dinv of block row r: the inverse of the row's diagonal block (found by scanning the row,
 // inverted in double from its upper triangle, stored as 3 rows of 4 in T), the
 // block-diagonal preconditioner of BlockedSparseMatrix::prepare_preconditioning.  A row
-// without a diagonal block gets Dinv = 0 and is counted in *missing.
+// without a diagonal block gets Dinv = 0 and is counted in flags[0]; flags[1]: the longest row.
 template <typename T>
 __global__ void k_block_jacobi_rows(int n_blocks, const int32_t* __restrict__ row_ptr, const int32_t* __restrict__ cols,
-                                    const T* __restrict__ vals, int64_t vs, T* __restrict__ Dinv, int* missing)
+                                    const T* __restrict__ vals, int64_t vs, T* __restrict__ Dinv, int* flags)
 {
     const int r = blockIdx.x * blockDim.x + threadIdx.x;
+    const int longest = __reduce_max_sync(0xffffffffu, r < n_blocks ? row_ptr[r + 1] - row_ptr[r] : 0);
+    if ((threadIdx.x & 31) == 0) atomicMax(flags + 1, longest);
     if (r >= n_blocks) return;
     int64_t k = -1;
     for (int64_t j = row_ptr[r], e = row_ptr[r + 1]; j < e; ++j)
@@ -36,7 +38,7 @@ __global__ void k_block_jacobi_rows(int n_blocks, const int32_t* __restrict__ ro
     T* o = Dinv + (int64_t)r * 12;
     if (k < 0) {
         for (int i = 0; i < 12; ++i) o[i] = T(0);
-        atomicAdd(missing, 1);
+        atomicAdd(flags, 1);
         return;
     }
     const double a = vals[k], b = vals[vs + k], c = vals[2 * vs + k], d = vals[4 * vs + k], e = vals[5 * vs + k],
@@ -50,7 +52,7 @@ __global__ void k_block_jacobi_rows(int n_blocks, const int32_t* __restrict__ ro
 }
 
 // The solver state at the start of the workspace: PcgState, then 4 ints ([0] counts the
-// rows without a diagonal block).
+// rows without a diagonal block, [1] is the length of the longest row).
 struct Header {
     PcgState st;
     int flags[4];
@@ -126,7 +128,7 @@ BcsrPcgResult run_bcsr_pcg(int n_blocks, const int32_t* row_ptr, const int32_t* 
         throw std::invalid_argument("bcsr_pcg: vals_stride " + std::to_string(vals_stride) +
                                     " is smaller than the number of blocks row_ptr[n_blocks] = " + std::to_string(nnzb));
 
-    // The completion tickets and the missing-diagonal counter must start at zero.
+    // The completion tickets and the set-up kernel's two integers must start at zero.
     Header h{};
     h.st.abs_tol = abs_tol;
     h.st.rel_tol = rel_tol;
@@ -146,7 +148,12 @@ BcsrPcgResult run_bcsr_pcg(int n_blocks, const int32_t* row_ptr, const int32_t* 
 
     launch_pcg_init_rhs<T>(B, b, s);
     ResidentPlan resident;
-    const bool one_launch = plan_pcg_resident<T>(n_blocks, nnzb, resident);
+    // Large float matrices with rows of very different lengths (Tet10: the longest is 2.3 times the mean)
+    // are streamed by the two launches: ms of 60 iterations in two launches and in one: 68 MB of values
+    // 3.14 and 1.76, 112.5 MB 4.50 and 4.74, 132.5 MB 5.12 and 5.52; even rows of 27 blocks, 117 MB:
+    // 4.49 and 2.72, 134 MB: 4.56 and 3.81.
+    const bool uneven = (int64_t)h.flags[1] * n_blocks > 2 * (int64_t)nnzb;
+    const bool one_launch = plan_pcg_resident<T>(n_blocks, nnzb, sizeof(T) == 4 && uneven, resident);
     if (one_launch) {
         launch_pcg_resident<T>(B, resident, s);
         ck(cudaMemcpyAsync(&h, hdr, sizeof(Header), cudaMemcpyDeviceToHost, s), "read state");

@@ -26,7 +26,7 @@
 //    blocks per SM (GB300: 152 x 8 = 1,216).  A device with room for more resident blocks
 //    than 4,096 is refused by run_bcsr_pcg before any launch.
 //  * What must be zero when the kernels start: the eight completion tickets of the
-//    reductions and the missing-diagonal counter.  Every call clears them on its stream
+//    reductions and the set-up kernel's two integers.  Every call clears them on its stream
 //    (cudaMemsetAsync / cudaMemcpyAsync into the array) before its first kernel.  Everything
 //    else in the array is written before it is read.
 #include "bcsr_pcg.h"

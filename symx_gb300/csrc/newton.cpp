@@ -1352,13 +1352,14 @@ SolverReturn solve_t(SolverImpl& I, const NewtonSettings& S, SolveStats& st, int
         B.staged.f64_sums = S.cg_fp64_partial_sums ? 1 : 0;
         B.la = S.cg_lookahead && I.staged.lookahead ? I.la32.p : nullptr;
     }
-    // One-launch PCG: with the matrix in shared memory where it fits (the options of the staged
+    // One-launch PCG: with the matrix in shared memory and L2 where it fits (the options of the staged
     // kernel, residual replacement, FP64 partial sums and look-ahead, keep that one), else the
     // staged kernel (float), else two launches per iteration.
     symxg::ResidentPlan resident;
     const bool staged_options =
         std::is_same<T, float>::value && (S.cg_residual_replacement > 0 || S.cg_fp64_partial_sums || S.cg_lookahead);
-    const bool use_resident = !staged_options && symxg::plan_pcg_resident<T>(I.n_blocks, I.nnzb, resident);
+    const bool use_resident =
+        !staged_options && symxg::plan_pcg_resident<T>(I.n_blocks, I.nnzb, std::is_same<T, float>::value, resident);
     T* du = V[0].p;
 
     if (S.linear_solver != LinearSolver::BDPCG) throw std::runtime_error("symx_gb300: only the BDPCG linear solver is implemented");
@@ -1675,7 +1676,7 @@ AdjointInfo adjoint_pcg_t(SolverImpl& I, const double* rhs, double* lambda, doub
     symxg::launch_pcg_init<T>(B, I.grad.p, s);
     bool done = false;
     symxg::ResidentPlan resident;
-    if (symxg::plan_pcg_resident<T>(I.n_blocks, I.nnzb, resident)) {
+    if (symxg::plan_pcg_resident<T>(I.n_blocks, I.nnzb, std::is_same<T, float>::value, resident)) {
         symxg::launch_pcg_resident<T>(B, resident, s);
         done = true;
     } else if constexpr (std::is_same<T, float>::value) {

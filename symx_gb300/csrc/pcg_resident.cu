@@ -270,7 +270,7 @@ __device__ __forceinline__ T group_row_product(int kb, int ke, int q, const I* c
 }
 
 // First row of block b of G: the rows are cut so that each block gets the same share of
-// blocks(row) + (mean blocks per row), so no block has more than 2 n / G + 1 rows.  One warp,
+// blocks(row) + (mean blocks per row), so no block has more than 2 n / G + 2 rows.  One warp,
 // 32-way search over row_ptr.
 __device__ __forceinline__ int block_first_row(int b, int G, int n, const int32_t* __restrict__ row_ptr)
 {
@@ -662,9 +662,9 @@ __global__ void __launch_bounds__(resident_threads<T>(), 1) k_pcg_resident(PcgBu
     }
 }
 
-// SM count and shared memory per block of the current device (looked up once per device).
+// SM count, shared memory per block and L2 of the current device (looked up once per device).
 struct DeviceLimits {
-    int sms = 0, smem = 0;
+    int sms = 0, smem = 0, l2 = 0;
 };
 template <typename K>
 void allow_smem(K kernel, int bytes)
@@ -688,6 +688,7 @@ DeviceLimits device_limits()
     if (coop) {
         cudaDeviceGetAttribute(&d.sms, cudaDevAttrMultiProcessorCount, dev);
         cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+        cudaDeviceGetAttribute(&d.l2, cudaDevAttrL2CacheSize, dev);
         d.smem = (optin - 4096) & ~15;  // less the kernel's static shared memory
         allow_smem(k_pcg_resident<float, 4>, d.smem);
         allow_smem(k_pcg_resident<float, 16>, d.smem);
@@ -700,21 +701,33 @@ DeviceLimits device_limits()
 
 }  // namespace
 
-// Every system whose state and bitmap fit is taken, up to about 170,000 rows in float and 85,000 in
-// double: with most of the matrix read from L2 the kernel still matches the staged one (148,877
-// rows: 29.3 us per iteration in both).
+// Every system whose state and bitmap fit is taken: on GB300 up to about 145,200 rows in float and 80,100
+// in double, with most of the matrix read from L2 or HBM at the end of the range.  Us per iteration, two
+// launches -> this: float, rows of 27 blocks, 90 MB of values 58 -> 20, 117 MB 73 -> 39, 134 MB 74 -> 57;
+// double, 79,507 rows of 15 blocks 79 -> 60, of 27 (150 MB) 116 -> 97.
+//
+// With values_in_l2 (the float solver; uneven rows in the stand-alone one) the values also have to stay in
+// L2 from one iteration to the next: the staged kernel, or two launches where the rows are too long
+// for its ring (Tet10), stream them from HBM with more loads in flight.  Us per iteration, those -> this,
+// by bytes of all values: 76 MB (Tet4, 140,556 rows) 28.4 -> 19.4, 103 (Tet10) 62.1 -> 54.0, 105 (Hex8)
+// 34.4 -> 29.1, 108 (Tet10) 62.1 -> 60.2, 110 (Hex8) 34.9 -> 33.5, 112 (Hex8) 36.8 -> 36.2, 112.5 (Tet10)
+// 64.0 -> 67.1, 114 (Hex8) 36.7 -> 38.1, 127 (Tet10) 73 -> 78, (Hex8) 38.6 -> 55.2.  The line is at 13/16
+// of L2 (110 of 135.5 MB).
 template <typename T>
-bool plan_pcg_resident(int n_blocks, int64_t nnzb, ResidentPlan& plan)
+bool plan_pcg_resident(int n_blocks, int64_t nnzb, bool values_in_l2, ResidentPlan& plan)
 {
     plan = ResidentPlan{};
     if (n_blocks <= 0 || nnzb <= 0) return false;
     const DeviceLimits d = device_limits();
     if (d.sms <= 0) return false;
+    if (values_in_l2 && 9 * (int64_t)sizeof(T) * nnzb > (int64_t)d.l2 / 16 * 13) return false;
     constexpr int max_threads = resident_threads<T>();
     // at least sixteen rows per block: fewer would only add sums to wait for (1,000 rows in double:
     // 7.4 us per iteration on 63, 76 or 125 blocks)
     const int64_t grid = std::min<int64_t>(std::min(d.sms, kMaxGrid), ((int64_t)n_blocks + 15) / 16);
-    const int64_t rows = ((int64_t)n_blocks + grid - 1) / grid, rows_max = 2 * (int64_t)n_blocks / grid + 4;
+    const int64_t rows = ((int64_t)n_blocks + grid - 1) / grid;
+    // no block has more rows than 2 n / grid + 2 (block_first_row), rounded up to four in the kernel
+    const int64_t rows_max = (2 * (int64_t)n_blocks / grid + 2 + 3) & ~(int64_t)3;
     const int64_t state = rows_max * (kStateValues * (int64_t)sizeof(T) + 4) + 64;
     const int64_t bitmap = ((int64_t)n_blocks + 31) / 32 * 8;
     if (state + bitmap + 64 > d.smem) return false;
@@ -748,8 +761,8 @@ void launch_pcg_resident(const PcgBuffers<T>& B, const ResidentPlan& plan, cudaS
     count_launch();
 }
 
-template bool plan_pcg_resident<float>(int, int64_t, ResidentPlan&);
-template bool plan_pcg_resident<double>(int, int64_t, ResidentPlan&);
+template bool plan_pcg_resident<float>(int, int64_t, bool, ResidentPlan&);
+template bool plan_pcg_resident<double>(int, int64_t, bool, ResidentPlan&);
 template void launch_pcg_resident<float>(const PcgBuffers<float>&, const ResidentPlan&, cudaStream_t);
 template void launch_pcg_resident<double>(const PcgBuffers<double>&, const ResidentPlan&, cudaStream_t);
 
