@@ -357,10 +357,11 @@ __global__ void __launch_bounds__(resident_threads<T>(), 1) k_pcg_resident(PcgBu
     const int G = gridDim.x, n = B.n_blocks;
     if (tid == 0) {
         st0 = *B.state;
-        // The solve runs on b / 2^k with |b| about 2^k, exactly: the sums over all rows, in float's range
-        // for float, then neither overflow nor vanish for any b that its type holds.
-        constexpr int limit = sizeof(T) == 4 ? 120 : 1000;
-        b_exponent = st0.bb > 0.0 && st0.bb < (double)INFINITY ? min(max(ilogb(st0.bb) / 2, -limit), limit) : 0;
+        // The solve runs on b / 2^k, exactly, with |b| / 2^k about 2^20: the sums over all rows, in float's
+        // range for float, then do not overflow for any b that its type holds, and r.r can fall by 2^-180
+        // (tolerances of 1e-27) before it vanishes.
+        constexpr int limit = sizeof(T) == 4 ? 126 : 1000;
+        b_exponent = st0.bb > 0.0 && st0.bb < (double)INFINITY ? min(max(ilogb(st0.bb) / 2 - 20, -limit), limit) : 0;
         st0.bb = scalbn(st0.bb, -2 * b_exponent);
     }
     if (tid == 64) sum_place(place);

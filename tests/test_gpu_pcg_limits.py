@@ -49,3 +49,16 @@ def test_scaled_right_hand_side(lib, dtype, power):
     x, info = _solve(rp, cols, vals, b * 2.0 ** power, dtype, abs_tol=0.0, rel_tol=1e-5)
     assert i0["converged"] == 1 and info["converged"] == 1 and info["n_iterations"] == i0["n_iterations"]
     assert np.array_equal(x, x0 * 2.0 ** power)
+
+
+@pytest.mark.parametrize("dtype", ["float32", "float64"])
+@pytest.mark.parametrize("scale", [2.0 ** -20, 1.0, 2.0 ** 10])
+def test_tight_relative_tolerances(lib, dtype, scale):
+    """The recursive residual goes on falling below the rounding of b; 1e-22 of it is in range for any b."""
+    n = 3000
+    rp, cols, vals = _laplace(n)
+    b = scale * np.random.default_rng(6).uniform(0.5, 1.0, 3 * n)
+    for rel_tol in (1e-18, 1e-22):
+        x, info = _solve(rp, cols, vals, b, dtype, abs_tol=0.0, rel_tol=rel_tol)
+        assert info["converged"] == 1 and info["found_indefiniteness"] == 0
+        assert info["error"] < rel_tol
