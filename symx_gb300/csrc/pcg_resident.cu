@@ -123,10 +123,10 @@ constexpr int kSetWords = kSums * (kLevel0Words + kLevel1Words);
 constexpr size_t kSumBytes = sizeof(Word) * 2 * kSetWords;
 static_assert(kSumBytes <= 2 * sizeof(double) * kResidentPartials, "the exchange words fit in the partials");
 
-// Waits are bounded: the first one of a block to run out of polls sets *abort (in shared memory), and
-// every other wait of the block then gives up within eight polls (looking at each poll, and in thread 0
-// for the exit, made an iteration of 21,000 rows in float 0.05 us longer).
-constexpr int kAbortMask = 7;
+// Waits are bounded: one that runs out of polls sets *abort (in shared memory).  Waits for rows that
+// begin after that give up at once, and the block leaves after the exchange of that iteration, so a block
+// spends at most three times the limit.  (Looking at the flag in every poll made an iteration of 9,000
+// rows 0.06 us longer; once per wait costs nothing measurable.)
 template <typename S>
 __device__ __forceinline__ bool poll_sums(const Word* w, bool mine, unsigned long long tag, S& v, long long max_polls,
                                           volatile int* abort)
@@ -140,8 +140,6 @@ __device__ __forceinline__ bool poll_sums(const Word* w, bool mine, unsigned lon
             }
         }
         if (!__any_sync(0xffffffffu, mine)) return true;
-        // a vote: the warp leaves together
-        if ((polls & kAbortMask) == kAbortMask && __any_sync(0xffffffffu, *abort)) return false;
     }
     *abort = 1;
     return false;
@@ -230,6 +228,9 @@ __device__ __forceinline__ double p_dot_q(double zw, double zq_pw, double pq, do
 {
     return fma(beta, fma(beta, pq, zq_pw), zw);
 }
+// 2^e, within T's normal numbers
+__device__ __forceinline__ void power_of_two(int e, float& x) { x = __int_as_float((127 + e) << 23); }
+__device__ __forceinline__ void power_of_two(int e, double& x) { x = __hiloint2double((1023 + e) << 20, 0); }
 __device__ __forceinline__ bool positive(FF a) { return a.hi > 0.f; }
 __device__ __forceinline__ bool positive(double a) { return a > 0.0; }
 
@@ -386,7 +387,9 @@ __global__ void __launch_bounds__(resident_threads<T>(), 1) k_pcg_resident(PcgBu
     for (int i = tid; i <= rows; i += threads) rp[i] = B.row_ptr[row0 + i];
     for (int j = tid; j < 3 * R; j += threads) sx[j] = sr[j] = sz[j] = sp[j] = sq[j] = sw[j] = T(0);
     __syncthreads();
-    const T to_unit = (T)scalbn(1.0, -b_exponent), from_unit = (T)scalbn(1.0, b_exponent);
+    T to_unit, from_unit;
+    power_of_two(-b_exponent, to_unit);
+    power_of_two(b_exponent, from_unit);
     for (int i = tid; i < rows; i += threads) {
         const int64_t g = row0 + i;
         Row4<T> r = ld4(B.r + 4 * g), z = ld4(B.z + 4 * g);
@@ -504,8 +507,9 @@ __global__ void __launch_bounds__(resident_threads<T>(), 1) k_pcg_resident(PcgBu
         // ---- z of the gathered columns
         auto wait_row = [&](int c) {
             Row4<T> z;
+            const long long limit = *abort ? 0 : max_polls;
             for (long long polls = 0; !read_row(zt, c, tag, z); ++polls)
-                if (polls >= max_polls || ((polls & kAbortMask) == kAbortMask && *abort)) {
+                if (polls >= limit) {
                     *abort = 1;
                     break;
                 }
