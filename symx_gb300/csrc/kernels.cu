@@ -383,11 +383,11 @@ struct ProjPairsCfg {
     // row stride of A and B: the four accesses of a round's blocks take 54.6 shared-memory
     // wavefronts with a stride of 31 and 30.0 with 41 (the least of 31 .. 48); with it and the
     // sharing of the listed matrices below, 5,940 Hessians went from 1,024 to 631 us
-    static constexpr int LD = N == 30 ? 41 : N + 1;
+    static constexpr int LD = 41;
     static constexpr int VS = (N + 3) / 4 * 4;  // row stride of V in the reconstruction (16-byte rows)
     static constexpr int NP = N / 2, NR = N - 1, NOFF = NP * (NP - 1) / 2, SLOTS = (NOFF + 31) / 32;
-    static constexpr int mat_elems = ((N * LD > N * VS ? N * LD : N * VS) + 3) / 4 * 4;  // rows of V: 16-byte aligned
-    static_assert(VS % 4 == 0 && mat_elems % 4 == 0, "row_dot loads 16 bytes");
+    static constexpr int mat_elems = (N * LD + 3) / 4 * 4;  // rows of V: 16-byte aligned
+    static_assert(VS <= LD && VS % 4 == 0 && mat_elems % 4 == 0, "row_dot loads 16 bytes");
     // dynamic shared memory: A and B per warp, (c, s) per warp, the offset table
     static constexpr size_t off_B = (size_t)warps * mat_elems * sizeof(float);
     static constexpr size_t off_CS = off_B + (size_t)warps * mat_elems * sizeof(float);
@@ -526,7 +526,7 @@ __global__ void __launch_bounds__(ProjPairsCfg<N>::warps * 32, ProjPairsCfg<N>::
     k_project_pd_pairs(float* __restrict__ H, int64_t count, int tile, float eps, int mirroring, int* not_converged,
                        const int64_t* __restrict__ sel)
 {
-    static_assert(N % 6 == 0 && N <= 30, "N a multiple of 6 up to 30 (3 x 3 blocks, pairs of indices)");
+    static_assert(N == 30, "the row stride is chosen for 30");
     using Cfg = ProjPairsCfg<N>;
     constexpr int W = Cfg::warps, LD = Cfg::LD, VS = Cfg::VS;
     constexpr int NP = Cfg::NP, NR = Cfg::NR, NOFF = Cfg::NOFF, SLOTS = Cfg::SLOTS, nb = N / 3;
@@ -1098,7 +1098,10 @@ constexpr int kStagedConsumerWarps = 7;
 constexpr int kStagedThreads = 32 * (kStagedConsumerWarps + 1);  // warp 0: producer
 constexpr int kStagedRowsPerWarp = 8;                             // one block row per quad of lanes
 constexpr int kStagedRows = kStagedRowsPerWarp * kStagedConsumerWarps;
-constexpr int kStagedMaxStages = 8;
+// Two stages where three would fit: the rest of the SM's memory caches the gathered vector.  Us per
+// iteration with three and with two: Tet4 64^3 43.4 and 42.1 (42.5 with two and three blocks per SM),
+// look-ahead 66.7 and 61.7, Hex8 64^3 67.9 and 67.9.
+constexpr int kStagedStages = 2;
 // Bound of the drain waits (copies in flight before a block exits); the data waits use
 // B.staged.max_polls (wait_poll_limit()).
 constexpr long long kMaxBarrierPolls = kDefaultWaitPolls;
@@ -1165,37 +1168,28 @@ __host__ __device__ __forceinline__ size_t staged_stage_bytes(int cap, int stage
     return ((size_t)10 * cap * 4 + (size_t)(stage_rows + 4) * 4 + 127) / 128 * 128;
 }
 
-// Shared-memory layout of a staged block: full barriers, empty barriers (kStagedMaxStages
-// each), the chunk held by each ring slot, the per-chunk partial sums of the consumer warps
-// (kStagedPartSlots chunks in flight at most, with a count of the warps that stored theirs),
-// then the ring of stages.  The chunk slots and partials are used by the persistent kernel.
-constexpr int kStagedPartSlots = 2 * kStagedMaxStages;
-
-constexpr size_t kStagedHeaderBytes =
-    (16 * kStagedMaxStages + 4 * kStagedMaxStages + 4 * kStagedPartSlots +
-     8 * kStagedPartSlots * kStagedConsumerWarps + 127) / 128 * 128;
+// Shared-memory layout of a staged block: full barriers, empty barriers (kStagedStages each), then
+// the ring of stages.  The look-ahead kernel has more in front of its ring (la_shared).
+constexpr size_t kStagedHeaderBytes = (16 * kStagedStages + 127) / 128 * 128;
 struct StagedShared {
     uint64_t* full;
     uint64_t* empty;
-    int* chunk;        // [kStagedMaxStages] chunk index of the stage in each slot, -1: end of a pass
-    unsigned* wcount;  // [kStagedPartSlots] consumer warps that stored their partial
-    float2* wpart;     // [kStagedPartSlots][kStagedConsumerWarps] float-float warp partials
     unsigned char* stage0;
+    // look-ahead only
+    int* chunk;        // chunk index of the stage in each slot, -1: end of a pass
+    unsigned* wcount;  // per chunk in flight, the consumer warps that stored their partials
+    float2* wpart;     // per chunk in flight and warp, float-float partials
 };
 __device__ __forceinline__ StagedShared staged_shared(unsigned char* smem)
 {
-    StagedShared ss;
+    StagedShared ss{};
     ss.full = reinterpret_cast<uint64_t*>(smem);
-    ss.empty = ss.full + kStagedMaxStages;
-    ss.chunk = reinterpret_cast<int*>(smem + 16 * kStagedMaxStages);
-    ss.wcount = reinterpret_cast<unsigned*>(smem + 20 * kStagedMaxStages);
-    ss.wpart = reinterpret_cast<float2*>(smem + 20 * kStagedMaxStages + 4 * kStagedPartSlots);
+    ss.empty = ss.full + kStagedStages;
     ss.stage0 = smem + kStagedHeaderBytes;
     return ss;
 }
 __device__ __forceinline__ void staged_init_barriers(const StagedShared& ss, int stages)
 {
-    if (threadIdx.x < kStagedPartSlots) ss.wcount[threadIdx.x] = 0;
     if (threadIdx.x == 0) {
         for (int s = 0; s < stages; ++s) {
             mbar_init(smem_addr(&ss.full[s]), 1);
@@ -3090,11 +3084,8 @@ StagedSizes plan_staged_spmv(int n, const int32_t* rp, PcgBuffers<float>::Staged
         const size_t stage_bytes = staged_stage_bytes((int)cap, S);
         const int64_t budget =
             std::min<int64_t>(optin, per_sm_bytes / per_sm - 1024) - (int64_t)kStagedHeaderBytes - 1024;  // static smem
-        // Two stages where three would fit: the rest of the SM's memory caches the gathered vector.  PCG of
-        // 274,625 rows, 509 iterations: 22.1 ms with three stages, 21.4 with two (21.6 with two and three
-        // blocks per SM).
-        const int stages = (int)std::min<int64_t>(2, budget / (int64_t)stage_bytes);
-        if (stages < 2 || cap > (1 << 24)) continue;
+        constexpr int stages = kStagedStages;
+        if (stages * (int64_t)stage_bytes > budget || cap > (1 << 24)) continue;
         const size_t smem = kStagedHeaderBytes + (size_t)stages * stage_bytes;
         if (cudaFuncSetAttribute(k_pcg_spmv_staged, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
             cudaGetLastError();
