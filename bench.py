@@ -290,7 +290,8 @@ def run_ours(args):
     t_pcg_it = sum(x["pcg_solve_seconds"] for x in stats) / max(1, n_pcg_it)
     pcg_it_bytes = spmv_bytes + n3 * 4 + 160 * rf["n_block_rows"]
     if n_pcg_it:
-        kernel_name = "k_pcg_solve_staged (all PCG iterations in one cooperative launch; unit = one iteration)"
+        kernel_name = ("k_pcg_solve_staged (k_pcg_resident for systems that fit on chip; all PCG iterations in one "
+                       "cooperative launch; unit = one iteration)")
         roof_bytes, roof_t, roof_n, traffic_key = pcg_it_bytes, t_pcg_it, n_pcg_it, "k_pcg_solve_staged per iteration"
     else:
         kernel_name = "k_pcg_spmv_staged (PCG SpMV with fused direction update, live in the timed solves)"

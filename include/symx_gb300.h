@@ -197,7 +197,7 @@ int64_t symxg_launch_count(void);
  * sets it to the current value after reading it).  Either pointer may be NULL. */
 void symxg_device_memory(int64_t* current, int64_t* peak, int32_t reset_peak);
 
-/* Bound on the waits inside the staged PCG kernels (no counterpart in the reference, whose
+/* Bound on the waits inside the one-launch PCG kernels (no counterpart in the reference, whose
  * CPU solver never waits on another processor).  Every wait of those kernels on a
  * shared-memory stage or on the other blocks of the launch polls at most this many times;
  * when one gives up, the kernel stops its work, waits (with the default bound) for its own

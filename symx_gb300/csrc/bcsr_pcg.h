@@ -46,8 +46,9 @@ size_t bcsr_pcg_workspace_bytes(int n_blocks, unsigned partials_per_part)
 // sqrt(r.r / b.b) < abs_tol, when that error falls below rel_tol times its initial value, on
 // p.Ap <= 0, or after max_iterations.  `workspace` (16-byte aligned, `workspace_bytes` long)
 // holds every vector, the preconditioner, the reduction partials, the completion tickets and
-// the solver state; nothing is allocated.  The call reads the state back to the host between
-// chunks of iterations, so it returns with `s` synchronized.
+// the solver state; nothing is allocated.  The call reads the state back to the host after its one
+// launch (k_pcg_resident), or between chunks of iterations where the system is too large for that,
+// so it returns with `s` synchronized.
 template <typename T>
 BcsrPcgResult run_bcsr_pcg(int n_blocks, const int32_t* row_ptr, const int32_t* cols, const T* vals,
                            int64_t vals_stride, const T* b, T* x, double abs_tol, double rel_tol, int max_iterations,

@@ -871,8 +871,9 @@ __device__ __forceinline__ T half_warp_transpose_sum(const T (&a)[3], const T (&
 // y = A x (x and y with 3 values per block row, the C ABI layout).  Bound by the matrix's bytes, so a
 // thread block streams the blocks of its rows in storage order, two (in double four) per thread with
 // all their loads in flight, leaves the products in shared memory, and sums them with four lanes per
-// row.  (With half a warp per row, 16 lanes for about 15 blocks, too few loads were in flight: 4.0 M blocks in
-// float 45.1 us, now 35.0, or 4.8 TB/s; in double 145 and 124 us.)  What is left is the
+// row.  (With half a warp per row, 16 lanes for about 15 blocks, too few loads were in flight.  4.0 M blocks
+// back to back on the same inputs, part of which stays in L2: float 45.1 us, now 35.0; double 145 and
+// 124.  One product after a flush of L2, event times: float 55.9, now 46.2, 3.6 TB/s.)  What is left is the
 // chain of a chunk's loads, row pointers, then columns and values, then x.
 // In float, four per thread and eight blocks per SM take 38.8 us, two and sixteen spill (48 us).
 constexpr int kSpmvBlock = 128, kSpmvRows = kSpmvBlock / 4;

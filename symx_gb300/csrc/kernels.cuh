@@ -18,9 +18,9 @@ void note_device_free(int64_t bytes);
 int64_t device_bytes_current();
 int64_t device_bytes_peak(bool reset);
 
-// Polls after which a bounded wait of the staged PCG kernels (a shared-memory stage's
-// mbarrier, the persistent kernel's grid barrier) gives up and flags the solve
-// (PcgState::wait_failed).  Process-wide, read at each launch; the default is
+// Polls after which a bounded wait of the one-launch PCG kernels (a row or a block's sums in
+// k_pcg_resident; a shared-memory stage's mbarrier and the grid barrier of the staged kernels) gives
+// up and flags the solve (PcgState::wait_failed).  Process-wide, read at each launch; the default is
 // kDefaultWaitPolls.  A small value makes the waits run out on purpose, which is how the
 // error path is tested.  The drain of a block's bulk copies in flight before it exits always
 // uses the default, so a block never exits with a copy still writing its shared memory.

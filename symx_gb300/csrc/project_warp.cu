@@ -100,7 +100,8 @@ __device__ __forceinline__ void rotate_pair(double& app, double& apq, double& aq
 }
 
 // Parallel cyclic Jacobi on the symmetric M x M matrix A (shared memory, row stride LD, upper
-// triangle), M even, in the odd-even order: round 2 r rotates the neighbouring positions (0, 1),
+// triangle), M even, in the odd-even order (R. P. Brent, F. T. Luk, "The solution of singular-value and
+// symmetric eigenvalue problems on multiprocessor arrays", SIAM J. Sci. Stat. Comput. 6 (1985)): round 2 r rotates the neighbouring positions (0, 1),
 // (2, 3), ..., round 2 r + 1 the positions (1, 2), (3, 4), ..., and every rotation also swaps its
 // two positions, so after M rounds (a sweep) every pair of indices has met while the positions,
 // hence all addresses and registers, are the same two patterns throughout (the round-robin
@@ -652,8 +653,8 @@ __device__ __forceinline__ bool decompose_and_correct(T* __restrict__ h, const G
 // ---- one warp per matrix
 // Measured against Jacobi over all N indices (round-robin order, FP64 throughout in double): 16,687
 // 24 x 24 Hessians in float 891 -> 558 us (bound by issue and shared memory), 2,001 in double (70 %
-// indefinite) 3.74 -> 0.97 ms (bound by the FP64 pipe: the fullest quarter SM's is busy throughout, the
-// average one 57 %).  30 x 30 in float stays with that form (k_project_pd_pairs, 631 us for 5,940):
+// indefinite) 3.74 -> 0.97 ms (bound by the FP64 pipe: the fullest quarter SM's is busy for 81 % of the
+// time, the average one's for 47 %).  30 x 30 in float stays with that form (k_project_pd_pairs, 631 us for 5,940):
 // this one takes 449 us, but its other rounding moves the positions at which a Newton solve of
 // quadratic tetrahedra stops in mixed precision by up to 5e-9 of them.
 //
@@ -665,7 +666,8 @@ constexpr int kMaxTile = 512;
 template <typename T, int N>
 struct WarpCfg {
     static constexpr int warps = 8;
-    // 85 registers in float (four blocks per SM spill: 600 us where three take 558), 255 in double
+    // float: 80 registers, at most 24 bytes of spills (four blocks per SM spill more: 600 us where three
+    // take 558); double: 255
     static constexpr int min_blocks = sizeof(T) == 4 ? 3 : 1;
     static constexpr size_t smem = warps * GroupMem<T, N>::bytes;
 };
