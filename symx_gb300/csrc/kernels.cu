@@ -869,25 +869,49 @@ __device__ __forceinline__ T half_warp_transpose_sum(const T (&a)[3], const T (&
 }
 
 // y = A x (x and y with 3 values per block row, the C ABI layout).  Bound by the matrix's bytes, so a
-// thread block streams the blocks of its rows in storage order, two (in double four) per thread with
-// all their loads in flight, leaves the products in shared memory, and sums them with four lanes per
-// row.  (With half a warp per row, 16 lanes for about 15 blocks, too few loads were in flight.  4.0 M blocks
-// back to back on the same inputs, part of which stays in L2: float 45.1 us, now 35.0; double 145 and
-// 124.  One product after a flush of L2, event times: float 55.9, now 46.2, 3.6 TB/s.)  What is left is the
+// thread block streams the blocks of its rows in storage order, two per thread with all their loads
+// in flight, leaves the products in shared memory, and sums them with four lanes per row.  (With half
+// a warp per row, 16 lanes for about 15 blocks, too few loads were in flight.  4.0 M blocks back to
+// back on the same inputs, part of which stays in L2: float 45.1 us, now 35.0; double 152 and 126.
+// One product after a flush of L2, event times: float 55.9, now 46.2, 3.6 TB/s.)  What is left is the
 // chain of a chunk's loads, row pointers, then columns and values, then x.
-// In float, four per thread and eight blocks per SM take 38.8 us, two and sixteen spill (48 us).
+// In float, four per thread and eight blocks per SM take 38.8 us, two and sixteen spill (48 us); in
+// double, eight blocks per SM spill, and four per thread with four blocks per SM take 107 us where
+// this takes 45 (200,000 rows of one block).
+//
+// Double, rows of more than 24 blocks on average: half a warp per row after all.  The sums' additions
+// hold the FP64 pipe in warps that are mostly idle then (a chunk has fewer rows than a warp has
+// groups of four lanes).  Us streamed and by half warps: 100,000 rows of 20 blocks 87 and 99, of 24 94
+// and 99, of 27 106 and 97; 50,000 of 60 165 and 96; 20,000 of 120 151 and 86.
 constexpr int kSpmvBlock = 128, kSpmvRows = kSpmvBlock / 4;
 template <typename T, typename L>
-__global__ void __launch_bounds__(kSpmvBlock, sizeof(T) == 4 ? 12 : 4)
+__global__ void __launch_bounds__(kSpmvBlock, sizeof(T) == 4 ? 12 : 7)
     k_bcsr_spmv(int n_blocks, const int32_t* __restrict__ row_ptr, const int32_t* __restrict__ cols,
                 const T* __restrict__ vals, L lay, const T* __restrict__ x, T* __restrict__ y)
 {
-    constexpr int kSpmvUnroll = sizeof(T) == 4 ? 2 : 4, kSpmvChunk = kSpmvBlock * kSpmvUnroll;
+    constexpr int kSpmvUnroll = 2, kSpmvChunk = kSpmvBlock * kSpmvUnroll;
     __shared__ T prod[3][kSpmvChunk];
     const int tid = threadIdx.x, q = tid & 3;
     const int64_t st = lay.step();
     const int row0 = blockIdx.x * kSpmvRows, row_end = min(row0 + kSpmvRows, n_blocks), row = row0 + tid / 4;
     const int kb = row_ptr[row0], ke = row_ptr[row_end];
+    if constexpr (sizeof(T) == 8) {
+        if (row_end - row0 > 1 && ke - kb > 24 * (row_end - row0)) {
+            const int lane16 = tid & 15, half = (tid >> 4) & 1;
+            auto xv = [x](int c) { return Row4<T>{x[3 * (int64_t)c], x[3 * (int64_t)c + 1], x[3 * (int64_t)c + 2], T(0)}; };
+#pragma unroll 1
+            for (int base = row0 + 8 * (tid >> 5), end = base + 8; base < end; base += 4) {
+                const int rowA = base + half, rowB = base + 2 + half;
+                const bool vA = rowA < row_end, vB = rowB < row_end;
+                T a[3], b[3];
+                two_row_products<T>(rowA, vA, rowB, vB, lane16, row_ptr, cols, vals, lay, xv, a, b);
+                const T sum = half_warp_transpose_sum<T>(a, b, lane16);
+                const int idx = lane16 >> 1;  // 0..2 row A, 3..5 row B
+                if (!(lane16 & 1) && idx < 6 && (idx < 3 ? vA : vB)) y[3 * (int64_t)(idx < 3 ? rowA : rowB) + idx % 3] = sum;
+            }
+            return;
+        }
+    }
     const int mine_b = row < row_end ? row_ptr[row] : 0, mine_e = row < row_end ? row_ptr[row + 1] : 0;
     T a[3] = {T(0), T(0), T(0)};
     for (int64_t base = kb; base < ke; base += kSpmvChunk) {
