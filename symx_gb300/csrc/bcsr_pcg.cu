@@ -148,12 +148,8 @@ BcsrPcgResult run_bcsr_pcg(int n_blocks, const int32_t* row_ptr, const int32_t* 
 
     launch_pcg_init_rhs<T>(B, b, s);
     ResidentPlan resident;
-    // Large float matrices with rows of very different lengths (Tet10: the longest is 2.3 times the mean)
-    // are streamed by the two launches: ms of 60 iterations in two launches and in one: 68 MB of values
-    // 3.14 and 1.76, 112.5 MB 4.50 and 4.74, 132.5 MB 5.12 and 5.52; even rows of 27 blocks, 117 MB:
-    // 4.49 and 2.72, 134 MB: 4.56 and 3.81.
-    const bool uneven = (int64_t)h.flags[1] * n_blocks > 2 * (int64_t)nnzb;
-    const bool one_launch = plan_pcg_resident<T>(n_blocks, nnzb, sizeof(T) == 4 && uneven, resident);
+    const bool even = 4 * (int64_t)h.flags[1] * n_blocks <= 5 * (int64_t)nnzb;
+    const bool one_launch = plan_pcg_resident<T>(n_blocks, nnzb, even ? ResidentRows::even : ResidentRows::uneven, resident);
     if (one_launch) {
         launch_pcg_resident<T>(B, resident, s);
         ck(cudaMemcpyAsync(&h, hdr, sizeof(Header), cudaMemcpyDeviceToHost, s), "read state");

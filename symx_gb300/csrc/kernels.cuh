@@ -235,11 +235,13 @@ void launch_pcg_solve_persistent(const PcgBuffers<float>& B, cudaStream_t s);
 
 // All PCG iterations in one cooperative launch with the matrix rows held in shared memory
 // (k_pcg_resident), float or double, strided values: for systems whose vectors fit in the SMs'
-// shared memory together.  plan_pcg_resident returns false when they do not, or, with values_in_l2,
-// when the matrix values exceed 13/16 of L2 (the plan depends on the device and its arguments only).  The launch uses the first kResidentPartials entries of
+// shared memory together.  plan_pcg_resident returns false when they do not, or when the matrix is
+// so large that the other kernels stream it faster (the plan depends on the device and its arguments
+// only).  The launch uses the first kResidentPartials entries of
 // both halves of B.partials and all of B.p2 (cleared here), and ends like
 // launch_pcg_solve_persistent.
 constexpr int kResidentPartials = 4096;
+enum class ResidentRows { even, uneven };  // uneven: the longest row above 5/4 of the mean, or not known
 struct ResidentPlan {
     int grid = 0;  // 0: not planned
     int threads = 0;
@@ -247,7 +249,7 @@ struct ResidentPlan {
     int smem_bytes = 0;
 };
 template <typename T>
-bool plan_pcg_resident(int n_blocks, int64_t nnzb, bool values_in_l2, ResidentPlan& plan);
+bool plan_pcg_resident(int n_blocks, int64_t nnzb, ResidentRows row_lengths, ResidentPlan& plan);
 template <typename T>
 void launch_pcg_resident(const PcgBuffers<T>& B, const ResidentPlan& plan, cudaStream_t s);
 

@@ -1359,7 +1359,7 @@ SolverReturn solve_t(SolverImpl& I, const NewtonSettings& S, SolveStats& st, int
     const bool staged_options =
         std::is_same<T, float>::value && (S.cg_residual_replacement > 0 || S.cg_fp64_partial_sums || S.cg_lookahead);
     const bool use_resident =
-        !staged_options && symxg::plan_pcg_resident<T>(I.n_blocks, I.nnzb, std::is_same<T, float>::value, resident);
+        !staged_options && symxg::plan_pcg_resident<T>(I.n_blocks, I.nnzb, symxg::ResidentRows::uneven, resident);
     T* du = V[0].p;
 
     if (S.linear_solver != LinearSolver::BDPCG) throw std::runtime_error("symx_gb300: only the BDPCG linear solver is implemented");
@@ -1676,7 +1676,7 @@ AdjointInfo adjoint_pcg_t(SolverImpl& I, const double* rhs, double* lambda, doub
     symxg::launch_pcg_init<T>(B, I.grad.p, s);
     bool done = false;
     symxg::ResidentPlan resident;
-    if (symxg::plan_pcg_resident<T>(I.n_blocks, I.nnzb, std::is_same<T, float>::value, resident)) {
+    if (symxg::plan_pcg_resident<T>(I.n_blocks, I.nnzb, symxg::ResidentRows::uneven, resident)) {
         symxg::launch_pcg_resident<T>(B, resident, s);
         done = true;
     } else if constexpr (std::is_same<T, float>::value) {

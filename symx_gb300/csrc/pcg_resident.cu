@@ -333,7 +333,7 @@ constexpr int kSumWarps = kSums + 1;  // the exchange's warps (one per sum) and 
 //   * no fence: a tagged word is its own release, a block's sums are published after its product,
 //     hence after its reads of z, and z is overwritten only after every block's sums arrived.
 //
-// LPR lanes take one block row: 4 where the block's rows fill its threads, 16 for fewer rows
+// LPR lanes take one block row: 4 where the block's rows fill its threads, 16 for fewer or long rows
 // (a shorter chain of products per lane).  zt: 4 values per row, cleared before the launch.
 template <typename T, int LPR>
 __global__ void __launch_bounds__(resident_threads<T>(), 1) k_pcg_resident(PcgBuffers<T> B, Word* zt, int smem_bytes)
@@ -712,26 +712,29 @@ DeviceLimits device_limits()
 
 }  // namespace
 
-// Every system whose state and bitmap fit is taken: on GB300 up to about 145,200 rows in float and 80,100
-// in double, with most of the matrix read from L2 or HBM at the end of the range.  Us per iteration, two
-// launches -> this: float, rows of 27 blocks, 90 MB of values 58 -> 20, 117 MB 73 -> 39, 134 MB 74 -> 57;
-// double, 79,507 rows of 15 blocks 79 -> 60, of 27 (150 MB) 116 -> 97.
-//
-// With values_in_l2 (the float solver; uneven rows in the stand-alone one) the values also have to stay in
-// L2 from one iteration to the next: the staged kernel, or two launches where the rows are too long
-// for its ring (Tet10), stream them from HBM with more loads in flight.  Us per iteration, those -> this,
-// by bytes of all values: 76 MB (Tet4, 140,556 rows) 28.4 -> 19.4, 103 (Tet10) 62.1 -> 54.0, 105 (Hex8)
-// 34.4 -> 29.1, 108 (Tet10) 62.1 -> 60.2, 110 (Hex8) 34.9 -> 33.5, 112 (Hex8) 36.8 -> 36.2, 112.5 (Tet10)
-// 64.0 -> 67.1, 114 (Hex8) 36.7 -> 38.1, 127 (Tet10) 73 -> 78, (Hex8) 38.6 -> 55.2.  The line is at 13/16
-// of L2 (110 of 135.5 MB).
+// Every system whose state and bitmap fit is taken (on GB300 up to about 145,200 rows in float and 80,100
+// in double) while its values, as far as shared memory does not hold them, come from L2 or from HBM
+// faster here than in the kernels that stream them with more loads in flight.  Where that ends, by
+// bytes of all values:
+//   * float solver (staged kernel; two launches for Tet10, whose rows are too long for its ring), 13/16 of
+//     L2 (110 of 135.5 MB).  Us per iteration, those -> this: Tet4 76 MB 28.4 -> 19.4, Tet10 103 MB
+//     62.1 -> 54.0, 108 MB 62.1 -> 60.2, 112.5 MB 64.0 -> 67.1, 127 MB 73 -> 78; Hex8 105 MB
+//     34.4 -> 29.1, 110 MB 34.9 -> 33.5, 112 MB 36.8 -> 36.2, 114 MB 36.7 -> 38.1, 127 MB 38.6 -> 55.2.
+//   * Two launches otherwise; ms of 30 iterations.  Rows of uneven lengths (the longest above 5/4 of the
+//     mean: blocks finish apart), float 13/16 of L2: random 89 MB 1.12 -> 1.06, 117 MB 1.51 -> 1.40, 126 MB
+//     1.53 -> 1.58, 132 MB 1.44 -> 1.59.  Double 7/4 (237 MB): Tet10 158 MB 4.35 -> 4.12, random 233 MB
+//     3.28 -> 3.11, 347 MB 4.06 -> 4.14.
+//   * Even rows, float 15/8 (254 MB): 129 MB 2.39 -> 2.06, 243 MB 3.75 -> 3.14, 251 MB 3.75 -> 3.76, 321 MB
+//     4.21 -> 4.91.  Double 10 times L2: 642 MB 9.54 -> 8.89, 1280 MB 18.4 -> 17.7, 1696 MB 22.8 -> 23.7.
 template <typename T>
-bool plan_pcg_resident(int n_blocks, int64_t nnzb, bool values_in_l2, ResidentPlan& plan)
+bool plan_pcg_resident(int n_blocks, int64_t nnzb, ResidentRows row_lengths, ResidentPlan& plan)
 {
     plan = ResidentPlan{};
     if (n_blocks <= 0 || nnzb <= 0) return false;
     const DeviceLimits d = device_limits();
     if (d.sms <= 0) return false;
-    if (values_in_l2 && 9 * (int64_t)sizeof(T) * nnzb > (int64_t)d.l2 / 16 * 13) return false;
+    constexpr int64_t uneven16 = sizeof(T) == 4 ? 13 : 28, even16 = sizeof(T) == 4 ? 30 : 160;  // sixteenths of L2
+    if (9 * (int64_t)sizeof(T) * nnzb > d.l2 / 16 * (row_lengths == ResidentRows::even ? even16 : uneven16)) return false;
     constexpr int max_threads = resident_threads<T>();
     // at least sixteen rows per block: fewer would only add sums to wait for (1,000 rows in double:
     // 7.4 us per iteration on 63, 76 or 125 blocks)
@@ -743,7 +746,9 @@ bool plan_pcg_resident(int n_blocks, int64_t nnzb, bool values_in_l2, ResidentPl
     const int64_t bitmap = ((int64_t)n_blocks + 31) / 32 * 8;
     if (state + bitmap + 64 > d.smem) return false;
     plan.grid = (int)grid;
-    plan.lanes_per_row = rows * 16 <= max_threads ? 16 : 4;
+    // rows of 80 blocks and more keep 16 lanes busy however many there are (double, ms of 30 iterations with
+    // 4 lanes -> 16: 8,000 rows of 262 blocks 4.29 -> 3.09, of 104 1.46 -> 1.23, of 64 1.01 -> 1.05)
+    plan.lanes_per_row = rows * 16 <= max_threads || nnzb >= 80 * (int64_t)n_blocks ? 16 : 4;
     // room for a quarter more rows than the mean: blocks at the mesh's boundary have more, shorter
     // rows, and a second round of the product for a few of them would hold up every block
     const int64_t lanes = (rows + rows / 4) * plan.lanes_per_row;
@@ -772,8 +777,8 @@ void launch_pcg_resident(const PcgBuffers<T>& B, const ResidentPlan& plan, cudaS
     count_launch();
 }
 
-template bool plan_pcg_resident<float>(int, int64_t, bool, ResidentPlan&);
-template bool plan_pcg_resident<double>(int, int64_t, bool, ResidentPlan&);
+template bool plan_pcg_resident<float>(int, int64_t, ResidentRows, ResidentPlan&);
+template bool plan_pcg_resident<double>(int, int64_t, ResidentRows, ResidentPlan&);
 template void launch_pcg_resident<float>(const PcgBuffers<float>&, const ResidentPlan&, cudaStream_t);
 template void launch_pcg_resident<double>(const PcgBuffers<double>&, const ResidentPlan&, cudaStream_t);
 
