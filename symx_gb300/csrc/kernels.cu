@@ -872,82 +872,93 @@ __device__ __forceinline__ T half_warp_transpose_sum(const T (&a)[3], const T (&
 // thread block streams the blocks of its rows in storage order, two per thread with all their loads
 // in flight, leaves the products in shared memory, and sums them with four lanes per row.  (With half
 // a warp per row, 16 lanes for about 15 blocks, too few loads were in flight.  4.0 M blocks back to
-// back on the same inputs, part of which stays in L2: float 45.1 us, now 35.0; double 152 and 126.
+// back on the same inputs, part of which stays in L2: float 45.1 us, now 35.0; double 140 and 116.
 // One product after a flush of L2, event times: float 55.9, now 46.2, 3.6 TB/s.)  What is left is the
 // chain of a chunk's loads, row pointers, then columns and values, then x.
-// In float, four per thread and eight blocks per SM take 38.8 us, two and sixteen spill (48 us); in
-// double, eight blocks per SM spill, and four per thread with four blocks per SM take 107 us where
-// this takes 45 (200,000 rows of one block).
+// In float, four per thread and eight thread blocks per SM take 38.8 us, two and sixteen spill (48 us).
 //
-// Double, rows of more than 24 blocks on average: half a warp per row after all.  The sums' additions
-// hold the FP64 pipe in warps that are mostly idle then (a chunk has fewer rows than a warp has
-// groups of four lanes).  Us streamed and by half warps: 100,000 rows of 20 blocks 87 and 99, of 24 94
-// and 99, of 27 106 and 97; 50,000 of 60 165 and 96; 20,000 of 120 151 and 86.
-constexpr int kSpmvBlock = 128, kSpmvRows = kSpmvBlock / 4;
+// Double: rows of more than 24 blocks on average by half a warp per row after all, since the sums'
+// additions hold the FP64 pipe in warps that are mostly idle (a chunk has fewer rows than its warps
+// have groups of four lanes).  Us streamed and by half warps: 30,000 rows of 20 blocks 23.0 and 27.4, 10,000
+// of 24 11.4 and 12.0, 20,000 of 27 21.4 and 19.7, of 60 48.7 and 34.8.  16 rows per thread block, so that
+// a warp has its four rows in one pass; seven thread blocks per SM (eight spill).  Half a warp per row
+// throughout (32 rows per thread block of 256) and now: 1,000 rows of 15 blocks 4.1 and 3.4, 17,864
+// 10.9 and 10.1, 68,921 35.9 and 30.3; 50,000 of 27 45.0 and 43.6; 50,000 of one 26.4 and 11.9; 50,000 of
+// which every tenth has 30 and the others none 16.0 and 16.4.
+constexpr int kSpmvBlock = 128;
+template <typename T>
+constexpr int kSpmvRows = sizeof(T) == 4 ? 32 : 16;
 template <typename T, typename L>
 __global__ void __launch_bounds__(kSpmvBlock, sizeof(T) == 4 ? 12 : 7)
     k_bcsr_spmv(int n_blocks, const int32_t* __restrict__ row_ptr, const int32_t* __restrict__ cols,
                 const T* __restrict__ vals, L lay, const T* __restrict__ x, T* __restrict__ y)
 {
-    constexpr int kSpmvUnroll = 2, kSpmvChunk = kSpmvBlock * kSpmvUnroll;
-    __shared__ T prod[3][kSpmvChunk];
+    constexpr int kUnroll = 2, kBlock = kSpmvBlock, kChunk = kBlock * kUnroll;
+    __shared__ T prod[3][kChunk];
     const int tid = threadIdx.x, q = tid & 3;
     const int64_t st = lay.step();
-    const int row0 = blockIdx.x * kSpmvRows, row_end = min(row0 + kSpmvRows, n_blocks), row = row0 + tid / 4;
+    const int row0 = blockIdx.x * kSpmvRows<T>, row_end = min(row0 + kSpmvRows<T>, n_blocks), row = row0 + tid / 4;
     const int kb = row_ptr[row0], ke = row_ptr[row_end];
+    const bool sums = tid < 4 * kSpmvRows<T> && row < row_end;  // four lanes per row
+    const int mine_b = sums ? row_ptr[row] : 0, mine_e = sums ? row_ptr[row + 1] : 0;
     if constexpr (sizeof(T) == 8) {
         if (row_end - row0 > 1 && ke - kb > 24 * (row_end - row0)) {
             const int lane16 = tid & 15, half = (tid >> 4) & 1;
             auto xv = [x](int c) { return Row4<T>{x[3 * (int64_t)c], x[3 * (int64_t)c + 1], x[3 * (int64_t)c + 2], T(0)}; };
-#pragma unroll 1
-            for (int base = row0 + 8 * (tid >> 5), end = base + 8; base < end; base += 4) {
-                const int rowA = base + half, rowB = base + 2 + half;
-                const bool vA = rowA < row_end, vB = rowB < row_end;
-                T a[3], b[3];
-                two_row_products<T>(rowA, vA, rowB, vB, lane16, row_ptr, cols, vals, lay, xv, a, b);
-                const T sum = half_warp_transpose_sum<T>(a, b, lane16);
-                const int idx = lane16 >> 1;  // 0..2 row A, 3..5 row B
-                if (!(lane16 & 1) && idx < 6 && (idx < 3 ? vA : vB)) y[3 * (int64_t)(idx < 3 ? rowA : rowB) + idx % 3] = sum;
-            }
+            const int base = row0 + 4 * (tid >> 5), rowA = base + half, rowB = base + 2 + half;
+            const bool vA = rowA < row_end, vB = rowB < row_end;
+            T a[3], b[3];
+            two_row_products<T>(rowA, vA, rowB, vB, lane16, row_ptr, cols, vals, lay, xv, a, b);
+            const T sum = half_warp_transpose_sum<T>(a, b, lane16);
+            const int idx = lane16 >> 1;  // 0..2 row A, 3..5 row B
+            if (!(lane16 & 1) && idx < 6 && (idx < 3 ? vA : vB)) y[3 * (int64_t)(idx < 3 ? rowA : rowB) + idx % 3] = sum;
             return;
         }
     }
-    const int mine_b = row < row_end ? row_ptr[row] : 0, mine_e = row < row_end ? row_ptr[row + 1] : 0;
     T a[3] = {T(0), T(0), T(0)};
-    for (int64_t base = kb; base < ke; base += kSpmvChunk) {
-        int c[kSpmvUnroll];
-        T m[kSpmvUnroll][9];
+    bool empty = true;
+    for (int64_t base = kb; base < ke; base += kChunk) {
+        int c[kUnroll];
+        T m[kUnroll][9];
 #pragma unroll
-        for (int u = 0; u < kSpmvUnroll; ++u) {
-            const int64_t k = base + u * kSpmvBlock + tid;
+        for (int u = 0; u < kUnroll; ++u) {
+            const int64_t k = base + u * kBlock + tid;
             c[u] = k < ke ? cols[k] : -1;
         }
 #pragma unroll
-        for (int u = 0; u < kSpmvUnroll; ++u)
+        for (int u = 0; u < kUnroll; ++u)
             if (c[u] >= 0) {
-                const T* __restrict__ v = vals + lay.base(base + u * kSpmvBlock + tid);
+                const T* __restrict__ v = vals + lay.base(base + u * kBlock + tid);
 #pragma unroll
                 for (int i = 0; i < 9; ++i) m[u][i] = v[i * st];
             }
 #pragma unroll
-        for (int u = 0; u < kSpmvUnroll; ++u)
+        for (int u = 0; u < kUnroll; ++u)
             if (c[u] >= 0) {
                 const T* __restrict__ xc = x + 3 * (int64_t)c[u];
                 const T x0 = xc[0], x1 = xc[1], x2 = xc[2];
 #pragma unroll
                 for (int i = 0; i < 3; ++i)
-                    prod[i][u * kSpmvBlock + tid] = m[u][3 * i] * x0 + m[u][3 * i + 1] * x1 + m[u][3 * i + 2] * x2;
+                    prod[i][u * kBlock + tid] = m[u][3 * i] * x0 + m[u][3 * i + 1] * x1 + m[u][3 * i + 2] * x2;
             }
         __syncthreads();
-        const int e = (int)(min((int64_t)mine_e, base + kSpmvChunk) - base);
+        const int e = (int)(min((int64_t)mine_e, base + kChunk) - base);
         int k = (int)(max((int64_t)mine_b, base) - base) + q;
         // added as a half-warp's lanes would add up to 16 blocks: eight apart, four, two, one
-        for (; k < e; k += 16) {
+        auto sixteen = [&](int i) {
             const bool h4 = k + 4 < e, h8 = k + 8 < e, h12 = k + 12 < e;
+            return (prod[i][k] + (h8 ? prod[i][k + 8] : T(0))) +
+                   ((h4 ? prod[i][k + 4] : T(0)) + (h12 ? prod[i][k + 12] : T(0)));
+        };
+        if (sizeof(T) == 8 && empty && k < e) {  // an FP64 addition to zero holds the pipe like any other
 #pragma unroll
-            for (int i = 0; i < 3; ++i)
-                a[i] += (prod[i][k] + (h8 ? prod[i][k + 8] : T(0))) +
-                        ((h4 ? prod[i][k + 4] : T(0)) + (h12 ? prod[i][k + 12] : T(0)));
+            for (int i = 0; i < 3; ++i) a[i] = sixteen(i);
+            empty = false;
+            k += 16;
+        }
+        for (; k < e; k += 16) {
+#pragma unroll
+            for (int i = 0; i < 3; ++i) a[i] += sixteen(i);
         }
         __syncthreads();
     }
@@ -956,7 +967,7 @@ __global__ void __launch_bounds__(kSpmvBlock, sizeof(T) == 4 ? 12 : 7)
 #pragma unroll
         for (int i = 0; i < 3; ++i) a[i] += __shfl_xor_sync(0xffffffffu, a[i], o);
     }
-    if (row < row_end && q < 3) y[3 * (int64_t)row + q] = q == 0 ? a[0] : q == 1 ? a[1] : a[2];
+    if (sums && q < 3) y[3 * (int64_t)row + q] = q == 0 ? a[0] : q == 1 ? a[1] : a[2];
 }
 
 // Accumulator of the PCG dot products: float-float for the FP32 PCG, double for FP64.
@@ -3193,7 +3204,7 @@ void launch_bcsr_spmv(int n_blocks, const int32_t* row_ptr, const int32_t* cols,
                       const T* x, T* y, cudaStream_t s)
 {
     if (n_blocks <= 0) return;
-    const unsigned g = blocks_for(n_blocks, kSpmvRows);
+    const unsigned g = blocks_for(n_blocks, kSpmvRows<T>);
     if (vstride == kTiledBcsr)
         k_bcsr_spmv<T><<<g, kSpmvBlock, 0, s>>>(n_blocks, row_ptr, cols, vals, TiledBcsr{}, x, y);
     else
