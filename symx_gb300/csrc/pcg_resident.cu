@@ -359,7 +359,7 @@ __global__ void __launch_bounds__(resident_threads<T>(), 1) k_pcg_resident(PcgBu
     } ctl;
     const int tid = threadIdx.x, threads = blockDim.x, lane = tid & 31, warp = tid >> 5;
     const int G = gridDim.x, n = B.n_blocks;
-    if (tid == 0) {
+    if (tid == 96) {  // a warp of its own: the first three do what follows at the same time
         st0 = *B.state;
         // The solve runs on b / 2^k, exactly, with |b| / 2^k about 2^20: the sums over all rows, in float's
         // range for float, then do not overflow for any b that its type holds, and r.r can fall by 2^-180
