@@ -503,10 +503,9 @@ __device__ bool pairs_pd_shortcut(const float* __restrict__ A, float* __restrict
     // Cholesky (lower triangle, in place): lane i holds row i
     const float dmax = warp_allmax(lane < M ? B[lane * LD + lane] : 0.0f);
     const float tau = float(16 * M) * symxg_dev::UnitRoundoff<float>::value() * dmax;
-    if (lane < M) B[lane * LD + lane] -= fmaxf(eps, 0.0f);
-    __syncwarp();
+    const float shift = fmaxf(eps, 0.0f);
     for (int j = 0; j < M; ++j) {
-        const float d = B[j * LD + j];  // the same value in every lane
+        const float d = B[j * LD + j] - shift;  // the same value in every lane
         if (!(d > tau)) return false;
         const float r = 1.0f / sqrt(d);
         const bool mine = lane > j && lane < M;
